@@ -420,76 +420,188 @@ __global__ void pack_mask_kernel(long long nn, const uint8_t* __restrict__ dofma
   if (local) atomicAdd(count, local);
 }
 
-// ---- coarsest level: dense masked operator, Cholesky, explicit inverse ----
-__global__ void dense_from_stencil_kernel(Grid g, const double* __restrict__ A, const uint8_t* __restrict__ fix,
-                                          double* D) {
-  const int NX = g.nx + 1, NY = g.ny + 1, NZ = g.nz + 1;
+// ---- coarsest level: dense masked operator, explicit inverse ----
+// One thread per dense entry (row DOF i, column DOF j): the stencil entry when
+// the two nodes are neighbours, 0 otherwise and on fixed DOFs (1 on their
+// diagonal).  Also clears the inverse's status.  (A thread per node with its
+// 243 stencil entries in series took 20 to 50 us on the 45 to 160 nodes of a
+// coarsest level; a thread per entry takes about 4.)
+__global__ void __launch_bounds__(256) dense_from_stencil_kernel(Grid g, const double* __restrict__ A,
+                                                                 const uint8_t* __restrict__ fix, double* D,
+                                                                 int* status) {
+  const int NX = g.nx + 1, NY = g.ny + 1;
   const long long nn = g.nnode();
-  const long long n3 = 3 * nn;
-  // D is zeroed by the caller
-  for (long long n = blockIdx.x * (long long)blockDim.x + threadIdx.x; n < nn; n += (long long)gridDim.x * blockDim.x) {
-    const int iy = (int)(n % NY);
-    const long long r = n / NY;
-    const int ix = (int)(r % NX), iz = (int)(r / NX);
-    const int fi = fix[n];
-    for (int dz = -1; dz <= 1; ++dz)
-      for (int dx = -1; dx <= 1; ++dx)
-        for (int dy = -1; dy <= 1; ++dy) {
-          const int x = ix + dx, y = iy + dy, z = iz + dz;
-          if (x < 0 || x >= NX || y < 0 || y >= NY || z < 0 || z >= NZ) continue;
-          const long long m = g.nidx(x, y, z);
-          const int fm = fix[m];
-          for (int c = 0; c < 3; ++c)
-            for (int d = 0; d < 3; ++d) {
-              double v = A[(long long)stencil_k(jrel_of(dx, dy, dz), c, d) * nn + n];
-              if (((fi >> c) & 1) || ((fm >> d) & 1)) v = 0.0;
-              D[(3 * n + c) * n3 + 3 * m + d] = v;
-            }
-        }
-    for (int c = 0; c < 3; ++c)
-      if ((fi >> c) & 1) D[(3 * n + c) * n3 + 3 * n + c] = 1.0;
+  const int n3 = (int)(3 * nn);
+  if (blockIdx.x == 0 && threadIdx.x == 0) *status = 0;
+  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < (long long)n3 * n3;
+       t += (long long)gridDim.x * blockDim.x) {
+    const int i = (int)(t / n3), j = (int)(t - (long long)i * n3);
+    const int n = i / 3, c = i - 3 * n, m = j / 3, d = j - 3 * m;
+    const int ry = n / NY, sy = m / NY;
+    const int dy = (m - sy * NY) - (n - ry * NY), dz = sy / NX - ry / NX;
+    const int dx = (sy - (sy / NX) * NX) - (ry - (ry / NX) * NX);
+    double v = 0.0;
+    if (dx >= -1 && dx <= 1 && dy >= -1 && dy <= 1 && dz >= -1 && dz <= 1) {
+      const bool fixed = ((fix[n] >> c) & 1) || ((fix[m] >> d) & 1);
+      if (!fixed) v = A[(long long)stencil_k(jrel_of(dx, dy, dz), c, d) * nn + n];
+      else if (i == j) v = 1.0;
+    }
+    D[t] = v;
   }
 }
 
 // Dense inverse of the coarsest operator, entirely on the device (no host
 // round trip per set-up).  Gauss-Jordan without pivoting (SPD pivots stay
-// positive in exact arithmetic); if a pivot is not positive, the elimination
-// restarts from D with the diagonal raised by 1e-12, 1e-9, then 1e-6 times its
-// mean magnitude; if all of those fail too, Inv is the inverse diagonal of D.
-// *status = the number of shifted attempts used (0..3), or kGjFallback.
+// positive in exact arithmetic), in blocks of kGjBlk pivots, one launch each
+// (gj_block_step_kernel).  If a pivot is not positive, gj_retry_kernel repeats
+// the elimination from D with the diagonal raised by 1e-12, 1e-9, then 1e-6
+// times its mean magnitude; if all of those fail too, Inv is the inverse
+// diagonal of D.  *status = the number of shifted attempts used (0..3), or
+// kGjFallback.
 constexpr int kGjAttempts = 4;
 constexpr int kGjFallback = 4;
+constexpr int kGjRetry = -1;  // a block step met a non-positive pivot (until gj_retry_kernel has run)
+constexpr int kGjBlk = 32;
 
 __device__ __forceinline__ double gj_shift(const double* __restrict__ D, int n, int attempt) {
-  if (attempt == 0) return 0.0;
   double m = 0.0;
   for (int i = 0; i < n; ++i) m += fabs(D[(size_t)i * n + i]);
   m = fmax(m / n, 1e-300);
   return (attempt == 1 ? 1e-12 : (attempt == 2 ? 1e-9 : 1e-6)) * m;
 }
 
-__device__ __forceinline__ void gj_diag_fallback(const double* __restrict__ D, int n, double* Inv) {
-  for (long long t = threadIdx.x; t < (long long)n * n; t += blockDim.x) {
-    const int i = (int)(t / n), j = (int)(t % n);
-    const double d = D[(size_t)i * n + i];
-    Inv[t] = (i == j && d > 0.0) ? 1.0 / d : 0.0;
+// Pivots [32 kb, 32 kb + 32) of the elimination: block (J, I) of the grid writes
+// the 32 x 32 tile (I, J) of `out` from `in`.  With P = A_kk^-1 the sweep is
+//   A_kk <- P,  A_kJ <- P A_kJ,  A_Ik <- -A_Ik P,  A_IJ <- A_IJ - A_Ik P A_kJ,
+// so after the last block `out` holds the inverse (and out32, if given, its
+// rounding).  Every block inverts the diagonal tile for itself: its 32 pivots
+// in series, one block barrier each, are most of the step's 10 us, and a launch
+// that published P would only add its latency.  Rows and columns past n are the
+// identity's.  One block holding the whole matrix instead took 235 us at
+// n = 135 (entries in registers) and 8.5 ms at n = 336 (entries in L2, two
+// barriers and 900 KB of traffic per pivot); in blocks of 32 over all SMs they
+// take 53 and 115 us (193 us at n = 480).
+__global__ void __launch_bounds__(256) gj_block_step_kernel(int n, int kb, const double* __restrict__ in,
+                                                            double* __restrict__ out, float* out32, int* status) {
+  constexpr int B = kGjBlk, W = B + 2;  // rows stay 16-byte aligned
+  __shared__ __align__(16) double P[B][W], L[B][W], R[B][W];
+  __shared__ double rowk[2][B], colk[2][B];
+  const int I = blockIdx.y, J = blockIdx.x, tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  const bool last = kb == (int)gridDim.x - 1;
+  if (last && I > J) return;
+  auto at = [&](int bi, int bj, int r, int c) {
+    const int i = B * bi + r, j = B * bj + c;
+    return (i < n && j < n) ? in[(size_t)i * n + j] : (i == j ? 1.0 : 0.0);
+  };
+  double a[4], c[4];
+#pragma unroll
+  for (int r = 0; r < 4; ++r) a[r] = at(kb, kb, ty + 8 * r, tx);
+#pragma unroll
+  for (int r = 0; r < 4; ++r) {
+    c[r] = at(I, J, ty + 8 * r, tx);
+    L[ty + 8 * r][tx] = at(I, kb, ty + 8 * r, tx);
+    R[ty + 8 * r][tx] = at(kb, J, ty + 8 * r, tx);
+  }
+  bool bad = false;
+#pragma unroll
+  for (int kr = 0; kr < 4; ++kr)
+#pragma unroll
+    for (int kw = 0; kw < 8; ++kw) {
+      const int k = 8 * kr + kw, buf = k & 1;
+      if (ty == kw) rowk[buf][tx] = a[kr];
+      if (tx == k) {
+#pragma unroll
+        for (int r = 0; r < 4; ++r) colk[buf][ty + 8 * r] = a[r];
+      }
+      __syncthreads();
+      const double p = rowk[buf][k], g = rowk[buf][tx];
+      bad = bad || !(p > 0.0);
+      const double pk = 1.0 / p;
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        const double f = colk[buf][ty + 8 * r] * pk;
+        a[r] = tx == k ? (ty + 8 * r == k ? pk : -f) : a[r] - f * g;
+      }
+      if (ty == kw) a[kr] = tx == k ? pk : g * pk;
+    }
+  if (bad && threadIdx.x == 0 && I == kb && J == kb) *status = kGjRetry;
+#pragma unroll
+  for (int r = 0; r < 4; ++r) P[ty + 8 * r][tx] = a[r];
+  __syncthreads();
+  // rows ty + 8 r of X Y, column tx
+  auto product = [&](const double (*X)[W], const double (*Y)[W], double* y) {
+#pragma unroll
+    for (int r = 0; r < 4; ++r) y[r] = 0.0;
+#pragma unroll 8
+    for (int m = 0; m < B; m += 2) {
+      const double y0 = Y[m][tx], y1 = Y[m + 1][tx];
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        const double2 x = *reinterpret_cast<const double2*>(&X[ty + 8 * r][m]);
+        y[r] = fma(x.y, y1, fma(x.x, y0, y[r]));
+      }
+    }
+  };
+  double v[4];
+  if (I == kb && J == kb) {
+#pragma unroll
+    for (int r = 0; r < 4; ++r) v[r] = a[r];
+  } else if (J == kb) {
+    product(L, P, v);
+#pragma unroll
+    for (int r = 0; r < 4; ++r) v[r] = -v[r];
+  } else {
+    product(P, R, v);
+    if (I != kb) {
+      __syncthreads();
+#pragma unroll
+      for (int r = 0; r < 4; ++r) R[ty + 8 * r][tx] = v[r];
+      __syncthreads();
+      product(L, R, v);
+#pragma unroll
+      for (int r = 0; r < 4; ++r) v[r] = c[r] - v[r];
+    }
+  }
+  // the last step computes the tiles on and above the diagonal and mirrors them:
+  // rounding would leave the two halves apart by eps times the condition number,
+  // and CG needs a symmetric preconditioner
+  if (last && I == J) {
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < 4; ++r) P[ty + 8 * r][tx] = v[r];
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < 4; ++r) v[r] = 0.5 * (v[r] + P[tx][ty + 8 * r]);
+  }
+#pragma unroll
+  for (int r = 0; r < 4; ++r) {
+    const int i = B * I + ty + 8 * r, j = B * J + tx;
+    if (i < n && j < n) {
+      out[(size_t)i * n + j] = v[r];
+      if (out32) out32[(size_t)i * n + j] = (float)v[r];
+      if (last && I != J) {
+        out[(size_t)j * n + i] = v[r];
+        if (out32) out32[(size_t)j * n + i] = (float)v[r];
+      }
+    }
   }
 }
 
-// One block.  When `in_smem`, the working matrix lives in dynamic shared
-// memory (n <= 160), else in Inv.  Each pivot step copies row k and column k
-// aside, then updates every entry in one pass over the matrix, a warp per row
-// (two barriers per step).
-__global__ void __launch_bounds__(1024) dense_gj_inverse_kernel(int n, const double* __restrict__ D, double* Inv,
-                                                                int in_smem, int* status) {
-  extern __shared__ double sA[];  // [n * n if in_smem] [row k: n] [column k: n]
+// The attempts with a raised diagonal, after a block step met a non-positive
+// pivot (one block; returns at once otherwise).  The working matrix lives in
+// Inv; each pivot step copies row k and column k aside, then updates every
+// entry in one pass over the matrix, a warp per row (two barriers per step).
+__global__ void __launch_bounds__(1024) gj_retry_kernel(int n, const double* __restrict__ D, double* Inv,
+                                                        float* inv32, int* status) {
+  if (*status != kGjRetry) return;
+  extern __shared__ double sA[];  // [row k: n] [column k: n]
   const long long nn = (long long)n * n;
-  double* A = in_smem ? sA : Inv;
-  double* rowk = sA + (in_smem ? nn : 0);
+  double* A = Inv;
+  double* rowk = sA;
   double* colk = rowk + n;
   __shared__ int bad;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
-  int attempt = 0;
+  int attempt = 1;
   for (; attempt < kGjAttempts; ++attempt) {
     const double shift = gj_shift(D, n, attempt);
     for (long long t = threadIdx.x; t < nn; t += blockDim.x) A[t] = D[t] + ((t % (n + 1)) == 0 ? shift : 0.0);
@@ -520,110 +632,13 @@ __global__ void __launch_bounds__(1024) dense_gj_inverse_kernel(int n, const dou
     __syncthreads();  // every thread has read `bad` before thread 0 resets it
     if (!failed) break;
   }
-  if (attempt == kGjAttempts) {
-    gj_diag_fallback(D, n, Inv);
-  } else if (in_smem) {
-    for (long long t = threadIdx.x; t < nn; t += blockDim.x) Inv[t] = A[t];
-  }
-  if (threadIdx.x == 0) *status = attempt == kGjAttempts ? kGjFallback : attempt;
-}
-
-// Gauss-Jordan inverse of a small SPD matrix (n <= 160) held in registers: one
-// block of 16 x 32 threads, thread (w, l) owns the 10 x 5 entries (w + 16 r,
-// l + 32 c).  Per pivot step the owners of row k and column k publish them in
-// shared memory (double-buffered, one barrier per step) and every thread
-// updates its entries in registers.  Same arithmetic, attempts and status as
-// dense_gj_inverse_kernel.
-constexpr int kGjRegMaxN = 160;
-
-__global__ void __launch_bounds__(512, 1) dense_gj_inverse_reg_kernel(int n, const double* __restrict__ D, double* Inv,
-                                                                      int* status) {
-  constexpr int R = 10, C = 5;
-  __shared__ double rowk[2][kGjRegMaxN], colk[2][kGjRegMaxN];
-  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-  double a[R][C];
-  int attempt = 0;
-  for (; attempt < kGjAttempts; ++attempt) {
-    const double shift = gj_shift(D, n, attempt);
-#pragma unroll
-    for (int r = 0; r < R; ++r)
-#pragma unroll
-      for (int c = 0; c < C; ++c) {
-        const int i = w + 16 * r, j = l + 32 * c;
-        a[r][c] = (i < n && j < n) ? D[(size_t)i * n + j] + (i == j ? shift : 0.0) : 0.0;
-      }
-    int bad = 0;  // the same in every thread: each reads the pivot from shared memory
-    for (int k = 0; k < n; ++k) {
-      const int buf = k & 1;
-      // owners of row k (warp k % 16, r = k / 16) and of column k (lane k % 32,
-      // c = k / 32) publish them; selects keep every index compile-time
-      if (w == (k & 15)) {
-        const int kr = k >> 4;
-#pragma unroll
-        for (int c = 0; c < C; ++c) {
-          double v = 0.0;
-#pragma unroll
-          for (int r = 0; r < R; ++r) v = (r == kr) ? a[r][c] : v;
-          rowk[buf][l + 32 * c] = v;
-        }
-      }
-      if (l == (k & 31)) {
-        const int kc = k >> 5;
-#pragma unroll
-        for (int r = 0; r < R; ++r) {
-          double v = 0.0;
-#pragma unroll
-          for (int c = 0; c < C; ++c) v = (c == kc) ? a[r][c] : v;
-          colk[buf][w + 16 * r] = v;
-        }
-      }
-      __syncthreads();
-      const double p = rowk[buf][k];
-      if (!(p > 0.0) && !bad) bad = k + 1;
-      const double pk = 1.0 / (p > 0.0 ? p : 1e-300);
-      double g[C];
-#pragma unroll
-      for (int c = 0; c < C; ++c) g[c] = rowk[buf][l + 32 * c];
-      // every entry: a_ij -= (a_ik / a_kk) a_kj (one FMA each); row k and
-      // column k are then overwritten by their owners
-#pragma unroll
-      for (int r = 0; r < R; ++r) {
-        const double f = colk[buf][w + 16 * r] * pk;
-#pragma unroll
-        for (int c = 0; c < C; ++c) a[r][c] = a[r][c] - f * g[c];
-      }
-      if (w == (k & 15)) {  // row k: a_kj / a_kk
-        const int kr = k >> 4;
-#pragma unroll
-        for (int r = 0; r < R; ++r)
-          if (r == kr) {
-#pragma unroll
-            for (int c = 0; c < C; ++c) a[r][c] = g[c] * pk;
-          }
-      }
-      if (l == (k & 31)) {  // column k: -a_ik / a_kk, and 1 / a_kk on the diagonal
-        const int kc = k >> 5;
-#pragma unroll
-        for (int c = 0; c < C; ++c)
-          if (c == kc) {
-#pragma unroll
-            for (int r = 0; r < R; ++r) a[r][c] = (w + 16 * r == k) ? pk : -(colk[buf][w + 16 * r] * pk);
-          }
-      }
+  for (long long t = threadIdx.x; t < nn; t += blockDim.x) {
+    if (attempt == kGjAttempts) {
+      const int i = (int)(t / n), j = (int)(t % n);
+      const double d = D[(size_t)i * n + i];
+      Inv[t] = (i == j && d > 0.0) ? 1.0 / d : 0.0;
     }
-    __syncthreads();  // the last step's buffers are read before the next attempt writes them
-    if (!bad) break;
-  }
-  if (attempt == kGjAttempts) {
-    gj_diag_fallback(D, n, Inv);
-  } else {
-#pragma unroll
-    for (int r = 0; r < R; ++r)
-#pragma unroll
-      for (int c = 0; c < C; ++c) {
-        const int i = w + 16 * r, j = l + 32 * c;
-        if (i < n && j < n) Inv[(size_t)i * n + j] = a[r][c];
-      }
+    if (inv32) inv32[t] = (float)Inv[t];
   }
   if (threadIdx.x == 0) *status = attempt == kGjAttempts ? kGjFallback : attempt;
 }

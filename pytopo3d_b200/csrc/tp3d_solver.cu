@@ -276,7 +276,7 @@ struct tp3d_solver {
   std::vector<double*> coef;  // Chebyshev coefficients per level (device)
   int nlev = 1;
   int cn = 0;  // coarsest dense size
-  double *cdense = nullptr, *cinv64 = nullptr;
+  double *cdense = nullptr, *cinv64 = nullptr, *cwork = nullptr;
   float* cinv32 = nullptr;
   int* cstatus = nullptr;
 
@@ -2097,6 +2097,7 @@ extern "C" int tp3d_solver_create(int nelx, int nely, int nelz, const double* KE
   if (s->nlev > 1) {
     s->cdense = s->alloc<double>((size_t)s->cn * s->cn);
     s->cinv64 = s->alloc<double>((size_t)s->cn * s->cn);
+    s->cwork = s->alloc<double>((size_t)s->cn * s->cn);
     if (mixed) s->cinv32 = s->alloc<float>((size_t)s->cn * s->cn);
     s->cstatus = s->alloc<int>(1);
   }
@@ -2300,31 +2301,31 @@ extern "C" int tp3d_solver_set_density(tp3d_solver* s, const double* rho, double
     s->fine_chosen = true;
   }
   if (int rc = fork_spectra(s, 0)) return rc;
-  // The coarsest inverse (one block) runs on a side stream while the level
-  // builds and the power iterations use the rest of the GPU; its status is read
-  // after both.
+  // The coarsest inverse runs on a side stream while the level builds and the
+  // power iterations use the rest of the GPU; its status is read after both.
   auto coarsest_gj = [&](cudaStream_t cs) -> int {
     const int L = s->nlev - 1;
     const int n = s->cn;
-    TP3D_CHECK(cudaMemsetAsync(s->cdense, 0, (size_t)n * n * sizeof(double), cs));
-    dense_from_stencil_kernel<<<s->grid_blocks(s->grids[L].nnode()), 256, 0, cs>>>(s->grids[L], s->A64[L], s->fix[L],
-                                                                                    s->cdense);
+    dense_from_stencil_kernel<<<(unsigned)(((long long)n * n + 255) / 256), 256, 0, cs>>>(
+        s->grids[L], s->A64[L], s->fix[L], s->cdense, s->cstatus);
     count_launch();
-    if (n <= kGjRegMaxN) {
-      dense_gj_inverse_reg_kernel<<<1, 512, 0, cs>>>(n, s->cdense, s->cinv64, s->cstatus);
+    // block steps alternate between the two buffers so that the last one ends in
+    // cinv64; cdense stays as it is for the retry
+    const int nb = (n + kGjBlk - 1) / kGjBlk;
+    const double* in = s->cdense;
+    for (int k = 0; k < nb; ++k) {
+      const bool last = k == nb - 1;
+      double* out = (nb - 1 - k) % 2 == 0 ? s->cinv64 : s->cwork;
+      gj_block_step_kernel<<<dim3((unsigned)nb, (unsigned)nb), 256, 0, cs>>>(n, k, in, out, last ? s->cinv32 : nullptr,
+                                                                             s->cstatus);
       count_launch();
-    } else {
-      const size_t smem = 2 * (size_t)n * sizeof(double);
-      if (smem > 48 * 1024)
-        if (int rc = ensure_dynamic_smem(dense_gj_inverse_kernel, smem)) return rc;
-      dense_gj_inverse_kernel<<<1, 1024, smem, cs>>>(n, s->cdense, s->cinv64, 0, s->cstatus);
-      count_launch();
+      in = out;
     }
-    if (mixed) {
-      convert_kernel<double, float><<<s->grid_blocks((long long)n * n), 256, 0, cs>>>((long long)n * n, s->cinv64,
-                                                                                      s->cinv32);
-      count_launch();
-    }
+    const size_t smem = 2 * (size_t)n * sizeof(double);
+    if (smem > 48 * 1024)
+      if (int rc = ensure_dynamic_smem(gj_retry_kernel, smem)) return rc;
+    gj_retry_kernel<<<1, 1024, smem, cs>>>(n, s->cdense, s->cinv64, s->cinv32, s->cstatus);
+    count_launch();
     TP3D_CHECK_LAUNCH();
     return TP3D_OK;
   };

@@ -699,3 +699,33 @@ def test_ritz_start_lowers_the_energy_of_the_initial_guess(P, prec):
     s0.set_density(to_flat(rho), 3.0)
     assert L.tp3d_solver_ritz_start(s0._h, F.data_ptr(), U.data_ptr(), Up.data_ptr(), 1) == _lib.TP3D_ERR_ARG
     s0.close()
+
+
+# The coarsest inverse's block elimination (32 pivots a step): coarsest sizes
+# below one block, on a block's edge, just past one, and of many blocks.  On a
+# two-level hierarchy CG takes 23 to 37 iterations here with the one-block
+# elimination it replaced, and as many with the blocks (bound: 2 more); a wrong
+# tile leaves the preconditioner unsymmetric.
+@pytest.mark.parametrize("prec", ["fp64", "mixed"])
+@pytest.mark.parametrize("dims,n,its", [((2, 2, 2), 24, 23), ((6, 6, 2), 96, 31), ((6, 4, 4), 108, 28),
+                                        ((12, 8, 8), 525, 37)])
+def test_coarsest_inverse_block_sizes(P, dims, n, its, prec):
+    from pytopo3d_b200._tensors import to_flat
+    from pytopo3d_b200.solver import HexSolver
+
+    nx, ny, nz = dims
+    KE = P.lk_H8(elem_size=1.0)
+    rho, free, fmask = _problem(nx, ny, nz, seed=n, lo=0.2)
+    s = HexSolver(nx, ny, nz, KE, fmask, precision=prec, max_levels=2, coarsest_max_dofs=3 if n < 500 else 600,
+                  rtol=1e-10)
+    s.set_density(to_flat(rho), 3.0)
+    F = O.build_force_vector(nx, ny, nz, fmask.size)
+    U = s.solve(torch.as_tensor(F).cuda()).cpu().numpy()
+    st = s.stats()
+    assert st["coarsest_dofs"] == n and st["coarsest_status"] == 0 and st["fp64_fallback"] == 0, st
+    assert s.last_iterations <= its + 2
+    K, _ = O.assemble_K(rho, KE, 3.0, nx, ny, nz)
+    U_ref = np.zeros(fmask.size)
+    U_ref[free] = spla.spsolve(K[free][:, free].tocsc(), F[free])
+    np.testing.assert_allclose(U, U_ref, rtol=0, atol=1e-8 * np.abs(U_ref).max())
+    s.close()
