@@ -470,37 +470,47 @@ __device__ __forceinline__ double gj_shift(const double* __restrict__ D, int n, 
   return (attempt == 1 ? 1e-12 : (attempt == 2 ? 1e-9 : 1e-6)) * m;
 }
 
+// 1 / p by Newton's iteration on the reciprocal from its FP32 rounding (the
+// relative error squares each time: 2^-24, 2^-48, then the FP64 rounding): the
+// division's latency is a third of the chain of pivots.
+__device__ __forceinline__ double gj_rcp(double p) {
+  if (!(p > 1e-30 && p < 1e30)) return 1.0 / p;
+  double r = (double)__frcp_rn((float)p);
+#pragma unroll
+  for (int k = 0; k < 2; ++k) r = fma(r, fma(-p, r, 1.0), r);
+  return r;
+}
+
 // Pivots [32 kb, 32 kb + 32) of the elimination: block (J, I) of the grid writes
-// the 32 x 32 tile (I, J) of `out` from `in`.  With P = A_kk^-1 the sweep is
-//   A_kk <- P,  A_kJ <- P A_kJ,  A_Ik <- -A_Ik P,  A_IJ <- A_IJ - A_Ik P A_kJ,
-// so after the last block `out` holds the inverse (and out32, if given, its
-// rounding).  Every block inverts the diagonal tile for itself: its 32 pivots
-// in series, one block barrier each, are most of the step's 10 us, and a launch
-// that published P would only add its latency.  Rows and columns past n are the
-// identity's.  One block holding the whole matrix instead took 235 us at
-// n = 135 (entries in registers) and 8.5 ms at n = 336 (entries in L2, two
-// barriers and 900 KB of traffic per pivot); in blocks of 32 over all SMs they
-// take 53 and 115 us (193 us at n = 480).
+// the 32 x 32 tile (I, J) of `out` from `in`; after the last block `out` holds
+// the inverse (and out32, if given, its rounding).  Rows and columns past n are
+// the identity's.  A tile's updates need the rows and columns of the pivots as
+// they stand, so every block carries the tiles (k, k), (k, J) and (I, k) through
+// the 32 pivots with its own, 4 entries of each per thread, one barrier per
+// pivot: the arithmetic is that of the elimination pivot by pivot.  (Inverting
+// the tile (k, k) and multiplying, A_IJ - A_Ik P A_kJ, is shorter but loses
+// accuracy with the condition of that tile: on nearly singular binary designs CG
+// took 10000 iterations instead of 1500.)
+// The pivots in series bound it, about 12 us a step with the launch: 64 us at
+// n = 135, 143 us at 336, 249 us at 480.  One block holding the whole matrix took
+// 235 us at n = 135 (entries in registers) and 8.5 ms at n = 336 (entries in L2,
+// two barriers and 900 KB of traffic per pivot).
 __global__ void __launch_bounds__(256) gj_block_step_kernel(int n, int kb, const double* __restrict__ in,
                                                             double* __restrict__ out, float* out32, int* status) {
-  constexpr int B = kGjBlk, W = B + 2;  // rows stay 16-byte aligned
-  __shared__ __align__(16) double P[B][W], L[B][W], R[B][W];
-  __shared__ double rowk[2][B], colk[2][B];
+  constexpr int B = kGjBlk;
+  __shared__ double rowA[2][B], rowB[2][B], colA[2][B], colC[2][B];
   const int I = blockIdx.y, J = blockIdx.x, tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-  const bool last = kb == (int)gridDim.x - 1;
-  if (last && I > J) return;
-  auto at = [&](int bi, int bj, int r, int c) {
-    const int i = B * bi + r, j = B * bj + c;
+  auto at = [&](int bi, int bj, int r) {
+    const int i = B * bi + ty + 8 * r, j = B * bj + tx;
     return (i < n && j < n) ? in[(size_t)i * n + j] : (i == j ? 1.0 : 0.0);
   };
-  double a[4], c[4];
-#pragma unroll
-  for (int r = 0; r < 4; ++r) a[r] = at(kb, kb, ty + 8 * r, tx);
+  double a[4], b[4], c[4], d[4];  // tiles (k, k), (k, J), (I, k), (I, J)
 #pragma unroll
   for (int r = 0; r < 4; ++r) {
-    c[r] = at(I, J, ty + 8 * r, tx);
-    L[ty + 8 * r][tx] = at(I, kb, ty + 8 * r, tx);
-    R[ty + 8 * r][tx] = at(kb, J, ty + 8 * r, tx);
+    a[r] = at(kb, kb, r);
+    b[r] = at(kb, J, r);
+    c[r] = at(I, kb, r);
+    d[r] = at(I, J, r);
   }
   bool bad = false;
 #pragma unroll
@@ -508,81 +518,42 @@ __global__ void __launch_bounds__(256) gj_block_step_kernel(int n, int kb, const
 #pragma unroll
     for (int kw = 0; kw < 8; ++kw) {
       const int k = 8 * kr + kw, buf = k & 1;
-      if (ty == kw) rowk[buf][tx] = a[kr];
+      if (ty == kw) {
+        rowA[buf][tx] = a[kr];
+        rowB[buf][tx] = b[kr];
+      }
       if (tx == k) {
 #pragma unroll
-        for (int r = 0; r < 4; ++r) colk[buf][ty + 8 * r] = a[r];
+        for (int r = 0; r < 4; ++r) {
+          colA[buf][ty + 8 * r] = a[r];
+          colC[buf][ty + 8 * r] = c[r];
+        }
       }
       __syncthreads();
-      const double p = rowk[buf][k], g = rowk[buf][tx];
+      const double p = rowA[buf][k], ga = rowA[buf][tx], gb = rowB[buf][tx];
       bad = bad || !(p > 0.0);
-      const double pk = 1.0 / p;
+      const double pk = gj_rcp(p);
 #pragma unroll
       for (int r = 0; r < 4; ++r) {
-        const double f = colk[buf][ty + 8 * r] * pk;
-        a[r] = tx == k ? (ty + 8 * r == k ? pk : -f) : a[r] - f * g;
+        const double f = colA[buf][ty + 8 * r] * pk, h = colC[buf][ty + 8 * r] * pk;
+        a[r] = tx == k ? -f : a[r] - f * ga;
+        b[r] = b[r] - f * gb;
+        c[r] = tx == k ? -h : c[r] - h * ga;
+        d[r] = d[r] - h * gb;
       }
-      if (ty == kw) a[kr] = tx == k ? pk : g * pk;
+      if (ty == kw) {
+        a[kr] = tx == k ? pk : ga * pk;
+        b[kr] = gb * pk;
+      }
     }
   if (bad && threadIdx.x == 0 && I == kb && J == kb) *status = kGjRetry;
 #pragma unroll
-  for (int r = 0; r < 4; ++r) P[ty + 8 * r][tx] = a[r];
-  __syncthreads();
-  // rows ty + 8 r of X Y, column tx
-  auto product = [&](const double (*X)[W], const double (*Y)[W], double* y) {
-#pragma unroll
-    for (int r = 0; r < 4; ++r) y[r] = 0.0;
-#pragma unroll 8
-    for (int m = 0; m < B; m += 2) {
-      const double y0 = Y[m][tx], y1 = Y[m + 1][tx];
-#pragma unroll
-      for (int r = 0; r < 4; ++r) {
-        const double2 x = *reinterpret_cast<const double2*>(&X[ty + 8 * r][m]);
-        y[r] = fma(x.y, y1, fma(x.x, y0, y[r]));
-      }
-    }
-  };
-  double v[4];
-  if (I == kb && J == kb) {
-#pragma unroll
-    for (int r = 0; r < 4; ++r) v[r] = a[r];
-  } else if (J == kb) {
-    product(L, P, v);
-#pragma unroll
-    for (int r = 0; r < 4; ++r) v[r] = -v[r];
-  } else {
-    product(P, R, v);
-    if (I != kb) {
-      __syncthreads();
-#pragma unroll
-      for (int r = 0; r < 4; ++r) R[ty + 8 * r][tx] = v[r];
-      __syncthreads();
-      product(L, R, v);
-#pragma unroll
-      for (int r = 0; r < 4; ++r) v[r] = c[r] - v[r];
-    }
-  }
-  // the last step computes the tiles on and above the diagonal and mirrors them:
-  // rounding would leave the two halves apart by eps times the condition number,
-  // and CG needs a symmetric preconditioner
-  if (last && I == J) {
-    __syncthreads();
-#pragma unroll
-    for (int r = 0; r < 4; ++r) P[ty + 8 * r][tx] = v[r];
-    __syncthreads();
-#pragma unroll
-    for (int r = 0; r < 4; ++r) v[r] = 0.5 * (v[r] + P[tx][ty + 8 * r]);
-  }
-#pragma unroll
   for (int r = 0; r < 4; ++r) {
     const int i = B * I + ty + 8 * r, j = B * J + tx;
+    const double v = I == kb ? (J == kb ? a[r] : b[r]) : (J == kb ? c[r] : d[r]);
     if (i < n && j < n) {
-      out[(size_t)i * n + j] = v[r];
-      if (out32) out32[(size_t)i * n + j] = (float)v[r];
-      if (last && I != J) {
-        out[(size_t)j * n + i] = v[r];
-        if (out32) out32[(size_t)j * n + i] = (float)v[r];
-      }
+      out[(size_t)i * n + j] = v;
+      if (out32) out32[(size_t)i * n + j] = (float)v;
     }
   }
 }
