@@ -317,3 +317,51 @@ def test_expired_barrier_wait_reaches_the_host(P, golden):
     bx, brho = P.optimality_criteria_update_projected(*args)
     np.testing.assert_allclose(bx, golden["oc_best_x"], rtol=1e-12, atol=1e-13)
     np.testing.assert_allclose(brho, golden["oc_best_rho"], rtol=1e-12, atol=1e-13)
+
+
+# The OC kernel walks the reference's path from a few evaluations (secant steps
+# between halvings of the multiplier): sizes at the edges of its 32 x 8 tiles and
+# of its planes per block, every filter radius class, multipliers far below the
+# first probe (spread: log-normal sensitivities), and targets that no multiplier
+# reaches from either side (the walk is left for the ordinary steps).
+@pytest.mark.parametrize("dims,rmin,spread,frac", [
+    ((8, 32, 7), 1.2, 1.0, 0.3), ((9, 33, 3), 2.3, 4.0, 0.4), ((17, 5, 21), 3.6, 1.0, 0.5), ((16, 31, 2), 4.4, 8.0, 0.3),
+    ((12, 14, 9), 5.5, 0.5, 0.45), ((13, 8, 15), 6.9, 2.0, 0.35), ((8, 9, 6), 0.9, 3.0, 0.3), ((24, 12, 13), 1.5, 2.0, -1.0),
+    ((24, 12, 13), 2.9, 2.0, 2.0)])
+def test_oc_walk_matches_oracle_path(P, dims, rmin, spread, frac):
+    from pytopo3d_b200.oc_update import OCWorkspace, oc_update_flat
+    from pytopo3d_b200._tensors import from_flat, to_flat, to_flat_mask, vec
+
+    nx, ny, nz = dims
+    shape = (ny, nx, nz)
+    beta, eta, move = 2.0, 0.5, 0.2
+    rng = np.random.default_rng(nx + 10 * ny)
+    solid = rng.uniform(size=shape) < 0.05
+    void = (rng.uniform(size=shape) < 0.05) & ~solid
+    free = ~(solid | void)
+    # below every candidate's volume all of them sit at x - move: from x < move they
+    # would instead fall as 1 / sqrt(lambda) towards 0, and the last steps' volumes
+    # differ by rounding only (1e-14), which decides no first step
+    x = rng.uniform(0.25 if frac < 0.0 else 0.1, 0.9, size=shape)
+    x[solid], x[void] = 1.0, 0.0
+    Ho, Hso = O.build_filter(nx, ny, nz, rmin)
+    _, rho, dp = O.build_physical_density(x, Ho, Hso, beta, eta, solid, void)
+    dc = -np.exp(spread * rng.normal(size=shape))
+    dv = O.apply_density_filter_chain_rule(free.astype(float), dp, Ho, Hso)
+    target = frac * rho[free].sum() + (1.0 - frac) * 0.7 * rho[free].sum()
+    if frac < 0.0:
+        target = 1e-3 * free.sum()  # below every candidate
+    elif frac > 1.0:
+        target = 1.01 * free.sum()  # above every candidate
+    steps, best, lo, hi = _oracle_bisection((x, dc, dv, move, target, Ho, Hso, beta, eta, free, solid, void), 80, 1e-8)
+    xo, rhoo = O.oc_update_projected(x, dc, dv, move, target, Ho, Hso, beta, eta, free, solid, void)
+    H, Hs = P.build_filter(nx, ny, nz, rmin)
+    xf = to_flat(x)
+    xn, rn = torch.empty_like(xf), torch.empty_like(xf)
+    st = oc_update_flat(H, xf, to_flat(dc), to_flat(dv), vec(Hs), to_flat_mask(solid), to_flat_mask(void), move, target,
+                        beta, eta, xn, rn, OCWorkspace(H)).cpu().numpy()
+    assert int(st[2]) == steps
+    assert st[0] == best and st[5] == lo and st[6] == hi
+    # the same multiplier: candidates to rounding, filtered densities to the filter's 1e-12
+    np.testing.assert_allclose(from_flat(xn, shape).cpu().numpy(), xo, rtol=0, atol=1e-14)
+    np.testing.assert_allclose(from_flat(rn, shape).cpu().numpy(), rhoo, rtol=0, atol=1e-12)
