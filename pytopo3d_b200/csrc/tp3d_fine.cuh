@@ -61,6 +61,7 @@ __device__ __forceinline__ EpiIn<T> fine_epi_load(int mode, const OpIO<T>& io, l
     case kModeChebStep: return epi_load<T, kModeChebStep>(io, i);
     case kModeDinvApply: return epi_load<T, kModeDinvApply>(io, i);
     case kModeChebStepDot: return epi_load<T, kModeChebStepDot>(io, i);
+    case kModeChebFirstDot: return epi_load<T, kModeChebFirstDot>(io, i);
     default: return EpiIn<T>{};
   }
 }
@@ -76,6 +77,7 @@ __device__ __forceinline__ void fine_epilogue(int mode, const OpIO<T>& io, long 
     case kModeChebFirst: op_epilogue<T, kModeChebFirst>(io, i, fx, kv, own, in, part); break;
     case kModeChebStep: op_epilogue<T, kModeChebStep>(io, i, fx, kv, own, in, part); break;
     case kModeChebStepDot: op_epilogue<T, kModeChebStepDot>(io, i, fx, kv, own, in, part); break;
+    case kModeChebFirstDot: op_epilogue<T, kModeChebFirstDot>(io, i, fx, kv, own, in, part); break;
     default: op_epilogue<T, kModeDinvApply>(io, i, fx, kv, own, in, part); break;
   }
 }
@@ -282,7 +284,7 @@ __global__ void __launch_bounds__(256, 2) fine_apply_kernel(const __grid_constan
     }
     __syncthreads();
   }
-  if (p.mode == kModeCgQ || p.mode == kModeChebStepDot) {
+  if (p.mode == kModeCgQ || p.mode == kModeChebStepDot || p.mode == kModeChebFirstDot) {
     part = block_sum(part, red);
     if (tid == 0) p.io.partials[blockIdx.y * gridDim.x + blockIdx.x] = part;
     if (p.io.fin_count)

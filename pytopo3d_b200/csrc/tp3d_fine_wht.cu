@@ -41,13 +41,16 @@ struct WhtShapes<double> {
 };
 
 // Epilogue modes that the one-barrier shapes run in the one-barrier kernel:
-// the plain apply, the residual, the CG product and the power-iteration step.
-// The Chebyshev and Jacobi steps (up to nine epilogue inputs per node) spill
+// the plain apply, the residual, the CG product, the power-iteration step and
+// the degree-1 smoother's step (256x128x128 loop body 50.8 ms, 51.7 with that one
+// in the two-barrier kernel).
+// The other Chebyshev and Jacobi steps (up to nine epilogue inputs per node) spill
 // in it under 64 registers per thread and measured faster in the two-barrier
 // kernel (128x64x64 SIMP step: 8.98 ms with this split, 9.10 ms with every
 // mode in the one-barrier kernel, 9.02 ms with none).
 constexpr bool wht1_mode(int mode) {
-  return mode == kModeApply || mode == kModeResid || mode == kModeCgQ || mode == kModeDinvApply;
+  return mode == kModeApply || mode == kModeResid || mode == kModeCgQ || mode == kModeDinvApply ||
+         mode == kModeChebFirstDot;
 }
 
 // dynamic shared memory of a launch of variant v
@@ -78,6 +81,7 @@ struct WhtVariant {
       case kModeChebFirst: return fn<kModeChebFirst>();
       case kModeChebStep: return fn<kModeChebStep>();
       case kModeChebStepDot: return fn<kModeChebStepDot>();
+      case kModeChebFirstDot: return fn<kModeChebFirstDot>();
       default: return fn<kModeDinvApply>();
     }
   }
@@ -107,7 +111,7 @@ template <typename T, class ESrc>
 bool wht_prepare(int v) {
   const int nthr = WhtShapes<T>::nthr[v];
   const int smem = (int)wht_kernel_smem<T>(v);
-  for (int mode = 0; mode <= kModeChebStepDot; ++mode)
+  for (int mode = 0; mode <= kModeChebFirstDot; ++mode)
     if (ensure_dynamic_smem(wht_fn<T, ESrc>(mode, v), smem) != TP3D_OK) return false;
   return true;
 }

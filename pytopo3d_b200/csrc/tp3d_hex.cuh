@@ -56,7 +56,9 @@ enum ApplyMode : int {
   kModeChebFirst = 4,  // d = c0 Dinv (b - K u); out = u + d
   kModeChebStep = 5,   // d = c1 d + c2 Dinv (b - K u); out = u + d
   kModeDinvApply = 6,  // out = Dinv K u (power iteration for lambda_max(Dinv K))
-  kModeChebStepDot = 7,  // Chebyshev step (first step when io.step == 0), and partials += b . out
+  kModeChebStepDot = 7,  // Chebyshev step, and partials += b . out
+  kModeChebFirstDot = 8,  // out = u + c0 Dinv (b - K u), and partials += b . out: the only step of a degree-1
+                          // smoother, whose direction nothing reads
 };
 
 // Inputs / outputs shared by every operator kernel.
@@ -73,7 +75,7 @@ struct OpIO {
   double* partials = nullptr;
   const int* done = nullptr;  // skip when *done != 0
   const int* gate = nullptr;  // skip when *gate == 0
-  // reductions (kModeCgQ, kModeChebStepDot): when fin_count is set, the last
+  // reductions (mode_reduces): when fin_count is set, the last
   // block finishes the reduction and applies finalize op fin_op to *fin
   PcgState* fin = nullptr;
   int fin_op = 0;
@@ -95,16 +97,16 @@ struct EpiIn {
 template <int MODE>
 __host__ __device__ constexpr bool epi_reads_b() {
   return MODE == kModeResid || MODE == kModeJacobi || MODE == kModeChebFirst || MODE == kModeChebStep ||
-         MODE == kModeChebStepDot;
+         MODE == kModeChebStepDot || MODE == kModeChebFirstDot;
 }
 template <int MODE>
 __host__ __device__ constexpr bool epi_reads_dinv() {
   return MODE == kModeJacobi || MODE == kModeChebFirst || MODE == kModeChebStep || MODE == kModeDinvApply ||
-         MODE == kModeChebStepDot;
+         MODE == kModeChebStepDot || MODE == kModeChebFirstDot;
 }
 template <int MODE>
 __host__ __device__ constexpr bool mode_reduces() {
-  return MODE == kModeCgQ || MODE == kModeChebStepDot;
+  return MODE == kModeCgQ || MODE == kModeChebStepDot || MODE == kModeChebFirstDot;
 }
 
 template <typename T, int MODE>
@@ -139,11 +141,13 @@ __device__ __forceinline__ void op_epilogue(const OpIO<T>& io, long long i, bool
     io.d[i] = dd;
     io.out[i] = own + dd;
   } else if (MODE == kModeChebStepDot) {
-    T dd;
-    if (io.step == 0) dd = fx ? T(0) : (T)io.coef[0] * in.dinv * (in.b - kv);
-    else dd = fx ? T(0) : (T)io.coef[2 * io.step] * in.d + (T)io.coef[2 * io.step + 1] * in.dinv * (in.b - kv);
+    const T dd = fx ? T(0) : (T)io.coef[2 * io.step] * in.d + (T)io.coef[2 * io.step + 1] * in.dinv * (in.b - kv);
     io.d[i] = dd;
     const T z = own + dd;
+    io.out[i] = z;
+    part += (double)in.b * (double)z;
+  } else if (MODE == kModeChebFirstDot) {
+    const T z = own + (fx ? T(0) : (T)io.coef[0] * in.dinv * (in.b - kv));
     io.out[i] = z;
     part += (double)in.b * (double)z;
   } else {  // kModeDinvApply

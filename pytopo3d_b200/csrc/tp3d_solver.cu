@@ -810,7 +810,7 @@ struct tp3d_solver {
         io.fin = state;
         io.fin_op = dot_op;
         io.fin_count = fin_count;
-        rc |= apply_level<T, kModeChebStepDot>(L, io);
+        rc |= s == 0 ? apply_level<T, kModeChebFirstDot>(L, io) : apply_level<T, kModeChebStepDot>(L, io);
       } else if (o.smoother == 1) {
         rc |= apply_level<T, kModeJacobi>(L, io);
       } else if (s == 0) {
@@ -898,7 +898,7 @@ struct tp3d_solver {
     fs.coef = cheb ? coef[L] : nullptr;
     fs.omega = (T)o.omega;
     fs.x0 = lv.x[0];
-    fs.d = cheb ? lv.d : nullptr;
+    fs.d = keeps_direction(L) ? lv.d : nullptr;
     return fs;
   }
 
@@ -913,6 +913,11 @@ struct tp3d_solver {
     if (L > 1 && o.deep_sweeps > 0) return o.deep_sweeps;
     return (L > 0 && o.coarse_sweeps > 0) ? o.coarse_sweeps : o.post_sweeps;
   }
+
+  // Whether a pre-smoothing step after the first reads level L's Chebyshev
+  // direction (a degree-1 smoother, the fine level's default, neither keeps nor
+  // reads one: 13 MB less per CG update and smoothing step at 128x64x64 in FP32).
+  bool keeps_direction(int L) const { return o.smoother != 1 && pre_sweeps(L) > 1; }
 
   // Level L (the last smoothed level) and the coarsest solve as one block
   // (deep_cycle_kernel); the restriction that produced b took the first
@@ -931,7 +936,7 @@ struct tp3d_solver {
       p.inv_smem = deep_inv_smem ? 1 : 0;
       p.b = b;
       p.x0 = lv.x[0];
-      p.d0 = o.smoother != 1 ? lv.d : nullptr;
+      p.d0 = keeps_direction(L) ? lv.d : nullptr;
       p.xout = lv.x[0];
       p.pre = pre_sweeps(L);
       p.post = post_sweeps(L);
@@ -982,7 +987,7 @@ struct tp3d_solver {
     p.cn = cn;
     p.b = b;
     p.x0 = la.x[0];
-    p.d0 = o.smoother != 1 ? la.d : nullptr;
+    p.d0 = keeps_direction(L) ? la.d : nullptr;
     p.xout = la.x[0];
     p.preA = pre_sweeps(L);
     p.postA = post_sweeps(L);
@@ -1051,10 +1056,10 @@ struct tp3d_solver {
     const bool cheb = o.smoother != 1;
     int cur = 0;
     if (!zero_done) {
-      count_bytes((cheb ? 4.0 : 3.0) * sizeof(T) * ndof);
+      count_bytes((keeps_direction(L) ? 4.0 : 3.0) * sizeof(T) * ndof);
       launch(L == 0 ? kPdlFine : kPdlCoarse, smooth_zero_kernel<T>, dim3(grid_blocks(ndof)), dim3(256), 0, ndof, b,
              (const T*)lv.dinv, (T)o.omega, (const double*)(cheb ? coef[L] : nullptr), lv.x[cur],
-             cheb ? lv.d : (T*)nullptr, done);
+             keeps_direction(L) ? lv.d : (T*)nullptr, done);
     }
     *rc |= smooth_steps<T>(L, 1, pre_sweeps(L) - 1, &cur, b, done);
     auto& lc = levels<T>()[L + 1];
@@ -1077,7 +1082,7 @@ struct tp3d_solver {
       fs.coef = cheb ? coef[L + 1] : nullptr;
       fs.omega = (T)o.omega;
       fs.x0 = lc.x[0];
-      fs.d = cheb ? lc.d : nullptr;
+      fs.d = keeps_direction(L + 1) ? lc.d : nullptr;
     }
     if (resid_fused) {
       auto fill = [&](auto& p) {
@@ -1088,7 +1093,7 @@ struct tp3d_solver {
         p.io.done = done;
       };
       count_bytes(2.0 * sizeof(T) * ndof + 81.0 * stencil_bytes<T>(L) * ndof + (double)gl.nnode() +
-                  (double)gn.nnode() + (fuse_first ? 4.0 : 1.0) * sizeof(T) * 3.0 * gn.nnode());
+                  (double)gn.nnode() + (fuse_first ? (keeps_direction(L + 1) ? 4.0 : 3.0) : 1.0) * sizeof(T) * 3.0 * gn.nnode());
       const dim3 grid((unsigned)gn.nnode());
       bool done16 = false;
       if constexpr (sizeof(T) == 4) {
@@ -1110,7 +1115,7 @@ struct tp3d_solver {
       }
     } else {
       count_bytes((double)sizeof(T) * ndof + (double)gn.nnode() +
-                  (fuse_first ? 4.0 : 1.0) * sizeof(T) * 3.0 * gn.nnode());
+                  (fuse_first ? (keeps_direction(L + 1) ? 4.0 : 3.0) : 1.0) * sizeof(T) * 3.0 * gn.nnode());
       launch(kPdlCoarse, restrict_kernel<T>, plane_grid((gn.nx + 1) * (gn.ny + 1), gn.nz + 1), dim3(256), 0, gl,
              gn, (const T*)lv.r, (const uint8_t*)fix[L + 1], lc.b, done, fs);
     }
@@ -1520,7 +1525,7 @@ struct tp3d_solver {
     io.fin_count = fin_count;
     int rc = fine<double, kModeCgQ>(io);
     const CoarseFirstStep<double> fs0 = first_step<double>(0);
-    count_bytes((fs0.x0 ? 9.0 : 6.0) * 8.0 * ndof);
+    count_bytes((fs0.x0 ? (fs0.d ? 9.0 : 8.0) : 6.0) * 8.0 * ndof);
     launch(kPdlFine, cg_update_kernel<double>, dim3(nb), dim3(256), 0, ndof, K.u, (const double*)K.p, K.r,
            (const double*)K.q, state, partials, (int)kFinRR, fin_count, fs0);
     bool dot_done = false;
@@ -1649,7 +1654,7 @@ struct tp3d_solver {
     io.fin_count = fin_count;
     int rc = fine<float, kModeCgQ>(io);
     const CoarseFirstStep<float> fs0 = first_step<float>(0);
-    count_bytes((fs0.x0 ? 9.0 : 6.0) * 4.0 * ndof);
+    count_bytes((fs0.x0 ? (fs0.d ? 9.0 : 8.0) : 6.0) * 4.0 * ndof);
     launch(kPdlFine, cg_update_kernel<float>, dim3(nb), dim3(256), 0, ndof, K.u, (const float*)K.p, K.r,
            (const float*)K.q, state, partials, (int)kFinRRMixed, fin_count, fs0);
     // reliable update (each kernel is also gated on state->update itself)
