@@ -144,6 +144,86 @@ __device__ __noinline__ void cl_pass(const Grid g, const __nv_bfloat16* S, int l
   for (int c = 0; c < 3; ++c) ypart[(qp * 3 + c) * kClPassNodes + nl] = y[c];
 }
 
+// Value v of own DOF i (node n) into buf[i] of every other CTA whose halo holds
+// node n (remote stores; the next cluster barrier publishes them).
+__device__ __forceinline__ void cl_push(int halo, int chunk, int rk, int C, float* buf, int n, int i, float v) {
+  namespace cg = cooperative_groups;
+  cg::cluster_group cl = cg::this_cluster();
+  const int r0 = n - halo < 0 ? 0 : (n - halo) / chunk;
+  const int r1 = min(C - 1, (n + halo) / chunk);
+  for (int r = r0; r <= r1; ++r)
+    if (r != rk) *cl.map_shared_rank(buf + i, (unsigned)r) = v;
+}
+
+// Entries [j0, j1) of a full-length array of 3 values per node, from the CTAs
+// that own them (`chunk` nodes each); a block barrier at the end.
+__device__ __noinline__ void cl_pull(float* a, int j0, int j1, int chunk, int rk) {
+  namespace cg = cooperative_groups;
+  cg::cluster_group cl = cg::this_cluster();
+  for (int j = j0 + (int)threadIdx.x; j < j1; j += kClThreads) {
+    const int owner = (j / 3) / chunk;
+    if (owner != rk) a[j] = *cl.map_shared_rank(a + j, (unsigned)owner);
+  }
+  __syncthreads();
+}
+
+__device__ __forceinline__ void cl_node_xyz(const Grid& g, int n, int* x, int* y, int* z) {
+  const int NY = g.ny + 1, NX = g.nx + 1;
+  *y = n % NY;
+  const int r = n / NY;
+  *x = r % NX;
+  *z = r / NX;
+}
+
+// The grid transfers run once each per launch, and their code is fetched anew
+// every time (from HBM at 128x64x64, where the solve's vectors turn L2 over: 6-7
+// us for each of three transfers there, under 3 us at 61x30x37), so one copy of
+// each, out of line, serves both levels: the launch takes 54 us at 128x64x64, 70
+// with a copy per level.  (Smoothing steps out of line too save nothing more there
+// and cost 0.3 us a step where L2 holds the code.)
+
+// Restriction of a level's residual r to the nodes [c0, c1) of the next level
+// (fixed DOFs fixc) into bc; a block barrier at the end.
+__device__ __noinline__ void cl_restrict(const Grid g, const Grid gcl, float* r, int nodes, int halo, int chunk, int rk,
+                                         int c0, int c1, const uint8_t* fixc, float* bc) {
+  // fine nodes that these coarse nodes read
+  const int FX = g.nx + 1, FY = g.ny + 1, CX = gcl.nx + 1, CY = gcl.ny + 1;
+  auto f = [&](int c) {
+    const int Iy = c % CY, q = c / CY;
+    return 2 * Iy + FY * (2 * (q % CX) + FX * 2 * (q / CX));
+  };
+  if (c1 > c0) cl_pull(r, 3 * max(0, f(c0) - halo), 3 * min(nodes, f(c1 - 1) + halo + 1), chunk, rk);
+  for (int n = c0 + (int)threadIdx.x; n < c1; n += kClThreads) {
+    int x, y, z;
+    cl_node_xyz(gcl, n, &x, &y, &z);
+    restrict_node<float, LdPlain>(g, gcl, r, fixc, bc, x, y, z);
+  }
+  __syncthreads();
+}
+
+// Prolongation of the next level's iterate xc (`cchunk` nodes per CTA) onto the
+// own range [lo, hi) of a level's iterate xf and the neighbours' halos; the
+// cluster barrier at the end publishes it.
+__device__ __noinline__ void cl_prolong(const Grid g, const Grid gcl, float* xc, int cchunk, float* xf,
+                                        const uint8_t* fix, int lo, int hi, int halo, int chunk, int rk, int C) {
+  namespace cg = cooperative_groups;
+  // coarse node range read by the own nodes: the coarse z-planes iz / 2 and
+  // iz / 2 + 1 of every fine plane iz in the range (the coarse base index of a
+  // fine node is not monotone in the node index, so the range is taken by whole
+  // planes)
+  const int FXY = (g.nx + 1) * (g.ny + 1), CXY = (gcl.nx + 1) * (gcl.ny + 1);
+  if (hi > lo)
+    cl_pull(xc, 3 * CXY * ((lo / FXY) >> 1), 3 * min((int)gcl.nnode(), CXY * (((hi - 1) / FXY >> 1) + 2)), cchunk, rk);
+  for (int n = lo + (int)threadIdx.x; n < hi; n += kClThreads) {
+    int x, y, z;
+    cl_node_xyz(g, n, &x, &y, &z);
+    prolong_node<float, LdPlain>(g, gcl, xc, fix, xf, x, y, z);
+#pragma unroll 1
+    for (int c = 0; c < 3; ++c) cl_push(halo, chunk, rk, C, xf, n, 3 * n + c, xf[3 * n + c]);
+  }
+  cg::this_cluster().sync();
+}
+
 __global__ void __launch_bounds__(kClThreads, 1) cluster_cycle_kernel(const __grid_constant__ ClusterParams p) {
   namespace cg = cooperative_groups;
   pdl_entry();
@@ -210,23 +290,8 @@ __global__ void __launch_bounds__(kClThreads, 1) cluster_cycle_kernel(const __gr
   for (int n = t; n < nB; n += kClThreads) B.fix[n] = p.fixB[n];
   for (int n = t; n < nC; n += kClThreads) fixC[n] = p.fixC[n];
   deep_copy_wait();
-  __syncthreads();
+  cl.sync();  // every CTA is staged before the first remote store reaches it
 
-  // entries [j0, j1) of a full-length array, from the CTAs that own them
-  auto pull = [&](float* a, int j0, int j1, int chunk) {
-    for (int j = j0 + t; j < j1; j += kClThreads) {
-      const int owner = (j / 3) / chunk;
-      if (owner != rk) a[j] = *cl.map_shared_rank(a + j, (unsigned)owner);
-    }
-  };
-  // value v of own DOF i (node n) of V into buf[i] of every other CTA whose
-  // halo holds node n (remote stores; the next cluster barrier publishes them)
-  auto push = [&](const ClLevel& V, float* buf, int n, int i, float v) {
-    const int r0 = n - V.halo < 0 ? 0 : (n - V.halo) / V.chunk;
-    const int r1 = min(C - 1, (n + V.halo) / V.chunk);
-    for (int r = r0; r <= r1; ++r)
-      if (r != rk) *cl.map_shared_rank(buf + i, (unsigned)r) = v;
-  };
   auto pass = [&](const ClLevel& V, int base, const float* xv) { cl_pass(V.g, V.S, V.lo, V.hi, base, xv, ypart); };
   auto psum = [&](int nl, int c) {
     return ((ypart[(0 * 3 + c) * kClPassNodes + nl] + ypart[(1 * 3 + c) * kClPassNodes + nl]) +
@@ -258,7 +323,7 @@ __global__ void __launch_bounds__(kClThreads, 1) cluster_cycle_kernel(const __gr
           out = own + dd;
         }
         V.xn[i] = out;
-        push(V, V.xn, n, i, out);
+        cl_push(V.halo, V.chunk, rk, C, V.xn, n, i, out);
       }
       if (base + kClPassNodes < V.hi) __syncthreads();
     }
@@ -281,55 +346,18 @@ __global__ void __launch_bounds__(kClThreads, 1) cluster_cycle_kernel(const __gr
     }
     cl.sync();
   };
-  // fine node range read by the restriction to coarse nodes [c0, c1)
-  auto fine_range = [&](const Grid& gf, const Grid& gc, int c0, int c1, int nf, int* f0, int* f1) {
-    const int FX = gf.nx + 1, FY = gf.ny + 1, CX = gc.nx + 1, CY = gc.ny + 1;
-    const int H = FX * FY + FY + 1;
-    auto f = [&](int c) {
-      const int Iy = c % CY, r = c / CY;
-      return 2 * Iy + FY * (2 * (r % CX) + FX * 2 * (r / CX));
-    };
-    *f0 = c1 > c0 ? max(0, f(c0) - H) : 0;
-    *f1 = c1 > c0 ? min(nf, f(c1 - 1) + H + 1) : 0;
-  };
-  // coarse node range read by the prolongation to fine nodes [n0, n1): the
-  // coarse z-planes iz / 2 and iz / 2 + 1 of every fine plane iz in the range
-  // (the coarse base index of a fine node is not monotone in the node index,
-  // so the range is taken by whole planes)
-  auto coarse_range = [&](const Grid& gf, const Grid& gc, int n0, int n1, int nc, int* c0, int* c1) {
-    const int FXY = (gf.nx + 1) * (gf.ny + 1), CXY = (gc.nx + 1) * (gc.ny + 1);
-    *c0 = n1 > n0 ? CXY * ((n0 / FXY) >> 1) : 0;
-    *c1 = n1 > n0 ? min(nc, CXY * (((n1 - 1) / FXY >> 1) + 2)) : 0;
-  };
-  auto node_xyz = [](const Grid& g, int n, int* x, int* y, int* z) {
-    const int NY = g.ny + 1, NX = g.nx + 1;
-    *y = n % NY;
-    const int r = n / NY;
-    *x = r % NX;
-    *z = r / NX;
-  };
-
   // ---- level A: pre-smoothing (step 0 was taken by the restriction) ----
   for (int s = 1; s < p.preA; ++s) smooth(A, s, false);
   residual(A);
   // ---- restriction A -> B, with B's first smoothing step ----
+  cl_restrict(p.gA, p.gB, A.r, nA, A.halo, A.chunk, rk, B.lo, B.hi, B.fix, B.b);
   {
-    int f0, f1;
-    fine_range(p.gA, p.gB, B.lo, B.hi, nA, &f0, &f1);
-    pull(A.r, 3 * f0, 3 * f1, A.chunk);
-    __syncthreads();
-    for (int n = B.lo + t; n < B.hi; n += kClThreads) {
-      int x, y, z;
-      node_xyz(p.gB, n, &x, &y, &z);
-      restrict_node<float, LdPlain>(p.gA, p.gB, A.r, B.fix, B.b, x, y, z);
-    }
-    __syncthreads();
     const float w = p.cheb ? (float)B.coef[0] : p.omega;
     for (int i = 3 * B.lo + t; i < 3 * B.hi; i += kClThreads) {
       const int li = i - 3 * B.lo;
       const float v = w * B.dinv[li] * B.b[i];
       B.x[i] = v;
-      push(B, B.x, i / 3, i, v);
+      cl_push(B.halo, B.chunk, rk, C, B.x, i / 3, i, v);
       if (p.cheb) B.d[li] = v;
     }
     cl.sync();
@@ -337,20 +365,11 @@ __global__ void __launch_bounds__(kClThreads, 1) cluster_cycle_kernel(const __gr
   // ---- level B: pre-smoothing, residual ----
   for (int s = 1; s < p.preB; ++s) smooth(B, s, false);
   residual(B);
-  // ---- restriction B -> coarsest, coarsest product, prolongation ----
+  // ---- restriction B -> coarsest, coarsest product ----
+  cl_restrict(p.gB, p.gC, B.r, nB, B.halo, B.chunk, rk, loC, hiC, fixC, bc);
+  cl.sync();
+  cl_pull(bc, 0, p.cn, Ly.chC, rk);
   {
-    int f0, f1;
-    fine_range(p.gB, p.gC, loC, hiC, nB, &f0, &f1);
-    pull(B.r, 3 * f0, 3 * f1, B.chunk);
-    __syncthreads();
-    for (int n = loC + t; n < hiC; n += kClThreads) {
-      int x, y, z;
-      node_xyz(p.gC, n, &x, &y, &z);
-      restrict_node<float, LdPlain>(p.gB, p.gC, B.r, fixC, bc, x, y, z);
-    }
-    cl.sync();
-    pull(bc, 0, p.cn, Ly.chC);
-    __syncthreads();
     // own rows of xc = Inv bc, a warp per row (FP64 accumulation)
     const int warp = t >> 5, lane = t & 31;
     for (int i = 3 * loC + warp; i < 3 * hiC; i += kClThreads / 32) {
@@ -361,36 +380,11 @@ __global__ void __launch_bounds__(kClThreads, 1) cluster_cycle_kernel(const __gr
       if (lane == 0) xc[i] = (float)acc;
     }
     cl.sync();
-    int c0, c1;
-    coarse_range(p.gB, p.gC, B.lo, B.hi, nC, &c0, &c1);
-    pull(xc, 3 * c0, 3 * c1, Ly.chC);
-    __syncthreads();
-    for (int n = B.lo + t; n < B.hi; n += kClThreads) {
-      int x, y, z;
-      node_xyz(p.gB, n, &x, &y, &z);
-      prolong_node<float, LdPlain>(p.gB, p.gC, xc, B.fix, B.x, x, y, z);
-#pragma unroll
-      for (int c = 0; c < 3; ++c) push(B, B.x, n, 3 * n + c, B.x[3 * n + c]);
-    }
-    cl.sync();
   }
-  // ---- level B: post-smoothing ----
+  // ---- prolongation, level B's post-smoothing, prolongation B -> A ----
+  cl_prolong(p.gB, p.gC, xc, Ly.chC, B.x, B.fix, B.lo, B.hi, B.halo, B.chunk, rk, C);
   for (int s = 0; s < p.postB; ++s) smooth(B, s, s == 0);
-  // ---- prolongation B -> A ----
-  {
-    int c0, c1;
-    coarse_range(p.gA, p.gB, A.lo, A.hi, nB, &c0, &c1);
-    pull(B.x, 3 * c0, 3 * c1, B.chunk);
-    __syncthreads();
-    for (int n = A.lo + t; n < A.hi; n += kClThreads) {
-      int x, y, z;
-      node_xyz(p.gA, n, &x, &y, &z);
-      prolong_node<float, LdPlain>(p.gA, p.gB, B.x, A.fix, A.x, x, y, z);
-#pragma unroll
-      for (int c = 0; c < 3; ++c) push(A, A.x, n, 3 * n + c, A.x[3 * n + c]);
-    }
-    cl.sync();
-  }
+  cl_prolong(p.gA, p.gB, B.x, B.chunk, A.x, A.fix, A.lo, A.hi, A.halo, A.chunk, rk, C);
   // ---- level A: post-smoothing, result ----
   for (int s = 0; s < p.postA; ++s) smooth(A, s, s == 0);
   // every access to another CTA's shared memory came before the last cluster

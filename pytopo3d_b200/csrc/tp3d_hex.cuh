@@ -601,7 +601,8 @@ __device__ __forceinline__ void prolong_node(const Grid& gf, const Grid& gc, con
   const int CX = gc.nx + 1, CY = gc.ny + 1;
   const long long n = iy + (long long)FY * (ix + (long long)FX * iz);
   const int f = fixf[n];
-  if (f == 7) return;
+  T* dst = xf + 3 * n;
+  const T d0 = dst[0], d1 = dst[1], d2 = dst[2];  // in flight with the coarse values
   const int oy = iy & 1, ox = ix & 1, oz = iz & 1;
   const int CXY = CX * CY;
   const int base = (iy >> 1) + CY * (ix >> 1) + CXY * (iz >> 1);
@@ -624,10 +625,9 @@ __device__ __forceinline__ void prolong_node(const Grid& gf, const Grid& gc, con
       }
     }
   }
-  T* dst = xf + 3 * n;
-  if (!(f & 1)) dst[0] += s0;
-  if (!(f & 2)) dst[1] += s1;
-  if (!(f & 4)) dst[2] += s2;
+  if (!(f & 1)) dst[0] = d0 + s0;
+  if (!(f & 2)) dst[1] = d1 + s1;
+  if (!(f & 4)) dst[2] = d2 + s2;
 }
 
 template <typename T>
