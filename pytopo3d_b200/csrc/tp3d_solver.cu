@@ -1121,7 +1121,7 @@ struct tp3d_solver {
     }
     T* xc = vcycle<T>(L + 1, lc.b, done, rc, fuse_first);
     count_bytes((double)sizeof(T) * 3.0 * gn.nnode() + 2.0 * sizeof(T) * ndof + (double)gl.nnode());
-    launch(L == 0 ? kPdlFine : kPdlCoarse, prolong_add_kernel<T>, plane_grid((gl.nx + 1) * (gl.ny + 1), gl.nz + 1),
+    launch(L == 0 ? kPdlFine : kPdlCoarse, prolong_add_kernel<T>, plane_grid((gl.nx + 1) * prolong_pairs(gl), gl.nz + 1),
            dim3(256), 0, gl, gn, (const T*)xc, (const uint8_t*)fix[L], lv.x[cur], done);
     const bool dot_here = dot_op >= 0 && o.smoother != 1 && post_sweeps(L) >= 1;
     *rc |= smooth_steps<T>(L, 0, post_sweeps(L), &cur, b, done, dot_here ? dot_op : -1);
