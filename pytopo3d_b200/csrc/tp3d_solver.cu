@@ -748,7 +748,11 @@ struct tp3d_solver {
         p.fix = fix[L];
         p.io = io;
         const long long nn = grids[L].nnode();
-        launch(kPdlCoarse, nm3_apply_kernel<float, MODE>, dim3(grid_blocks((nn + 9) / 10, 8)), dim3(256), 0, p);
+        if (int rc = ensure_dynamic_smem(nm3_apply_kernel<float, MODE>, kNM3Smem)) return rc;
+        constexpr int warps = kNM3Threads / 32;
+        const long long blocks = ((nn + 9) / 10 + warps - 1) / warps;  // ten nodes per warp
+        launch(kPdlCoarse, nm3_apply_kernel<float, MODE>, dim3((unsigned)std::min(blocks, 5LL * nsm)), dim3(kNM3Threads),
+               kNM3Smem, p);
         TP3D_CHECK_LAUNCH();
         return TP3D_OK;
       }
