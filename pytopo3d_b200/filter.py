@@ -18,7 +18,7 @@ import numpy as np
 import torch
 
 from . import _lib
-from ._tensors import device, like_input, to_flat, to_flat_mask, vec
+from ._tensors import device, like_input, to_flat, to_flat_mask_view, vec
 
 FLOAT_EPSILON = 1e-9
 
@@ -137,7 +137,7 @@ def build_physical_density(x, H, Hs, beta: float, eta: float, protected_solid, p
     xf = to_flat(x)
     Hs_d = vec(Hs)
     rf, rp, dp = torch.empty_like(xf), torch.empty_like(xf), torch.empty_like(xf)
-    project_flat(H, xf, Hs_d, beta, eta, to_flat_mask(protected_solid), to_flat_mask(protected_void),
+    project_flat(H, xf, Hs_d, beta, eta, to_flat_mask_view(protected_solid), to_flat_mask_view(protected_void),
                  rf, rp, dp)
     return like_input(rf, shape, x), like_input(rp, shape, x), like_input(dp, shape, x)
 

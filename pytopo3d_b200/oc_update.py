@@ -13,7 +13,7 @@ import numpy as np
 import torch
 
 from . import _lib
-from ._tensors import device, like_input, to_flat, to_flat_mask, vec
+from ._tensors import device, like_input, to_flat, to_flat_mask_view, vec
 from .filter import ConeFilter, _as_filter
 
 
@@ -55,8 +55,8 @@ def optimality_criteria_update_projected(x, dc_dx, dv_dx, move: float, target_fr
         raise ValueError("max_bisection_iterations must be at least 1")
     H = _as_filter(H)
     shape = tuple(x.shape)
-    solid, void = to_flat_mask(protected_solid), to_flat_mask(protected_void)
-    free = to_flat_mask(free_mask)
+    solid, void = to_flat_mask_view(protected_solid), to_flat_mask_view(protected_void)
+    free = to_flat_mask_view(free_mask)
     if solid is not None and void is not None:
         if not torch.equal(free.bool(), ~(solid.bool() | void.bool())):
             raise ValueError("free_mask must equal ~(protected_solid | protected_void)")
