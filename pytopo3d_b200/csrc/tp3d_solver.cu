@@ -777,10 +777,21 @@ struct tp3d_solver {
     p.S = levels<T>()[L].A;
     p.fix = fix[L];
     p.io = io;
-    if (split) launch(kPdlCoarse, stencil_apply4_kernel<T, MODE>, dim3(grid_blocks(4 * ndof)), dim3(256), 0, p);
-    else launch(kPdlCoarse, stencil_apply_kernel<T, MODE>, dim3(grid_blocks(ndof)), dim3(256), 0, p);
+    if (split) launch(pdl_class<T>(L), stencil_apply4_kernel<T, MODE>, dim3(grid_blocks(4 * ndof)), dim3(256), 0, p);
+    else launch(pdl_class<T>(L), stencil_apply_kernel<T, MODE>, dim3(grid_blocks(ndof)), dim3(256), 0, p);
     TP3D_CHECK_LAUNCH();
     return TP3D_OK;
+  }
+
+  // The programmatic-launch class of the kernels over level L: the fine operator's
+  // class for the fine level and for the FP64 cycle's small levels, whose kernels
+  // last little longer than a launch (32x16x16 loop bodies 10.95 to 10.5 ms, 48x24x24
+  // gradient 16.1 to 15.5).  On
+  // the larger coarse levels the early blocks cost more than they save (128x64x64
+  // FP64 +3%), and so they do on the mixed form's levels (61x30x37 +2%).
+  template <typename T>
+  int pdl_class(int L) const {
+    return L == 0 || (sizeof(T) == 8 && 3 * grids[L].nnode() <= o.split_dofs) ? kPdlFine : kPdlCoarse;
   }
 
   // bytes per stencil coefficient of level L >= 1 in precision T's cycle
@@ -1048,7 +1059,7 @@ struct tp3d_solver {
       if constexpr (sizeof(T) == 8) inv = cinv64;
       else inv = cinv32;
       count_bytes((double)sizeof(T) * cn * cn + 2.0 * sizeof(T) * cn);
-      launch(kPdlCoarse, dense_matvec_kernel<T>, dim3(std::max(1, std::min(cn / 8 + 1, nsm))), dim3(256), 0, cn, inv,
+      launch(pdl_class<T>(L), dense_matvec_kernel<T>, dim3(std::max(1, std::min(cn / 8 + 1, nsm))), dim3(256), 0, cn, inv,
              b, lv.x[0], done);
       return lv.x[0];
     }
@@ -1120,12 +1131,12 @@ struct tp3d_solver {
     } else {
       count_bytes((double)sizeof(T) * ndof + (double)gn.nnode() +
                   (fuse_first ? (keeps_direction(L + 1) ? 4.0 : 3.0) : 1.0) * sizeof(T) * 3.0 * gn.nnode());
-      launch(kPdlCoarse, restrict_kernel<T>, plane_grid((gn.nx + 1) * (gn.ny + 1), gn.nz + 1), dim3(256), 0, gl,
+      launch(pdl_class<T>(L + 1), restrict_kernel<T>, plane_grid((gn.nx + 1) * (gn.ny + 1), gn.nz + 1), dim3(256), 0, gl,
              gn, (const T*)lv.r, (const uint8_t*)fix[L + 1], lc.b, done, fs);
     }
     T* xc = vcycle<T>(L + 1, lc.b, done, rc, fuse_first);
     count_bytes((double)sizeof(T) * 3.0 * gn.nnode() + 2.0 * sizeof(T) * ndof + (double)gl.nnode());
-    launch(L == 0 ? kPdlFine : kPdlCoarse, prolong_add_kernel<T>, plane_grid((gl.nx + 1) * prolong_pairs(gl), gl.nz + 1),
+    launch(pdl_class<T>(L), prolong_add_kernel<T>, plane_grid((gl.nx + 1) * prolong_pairs(gl), gl.nz + 1),
            dim3(256), 0, gl, gn, (const T*)xc, (const uint8_t*)fix[L], lv.x[cur], done);
     const bool dot_here = dot_op >= 0 && o.smoother != 1 && post_sweeps(L) >= 1;
     *rc |= smooth_steps<T>(L, 0, post_sweeps(L), &cur, b, done, dot_here ? dot_op : -1);
