@@ -122,9 +122,8 @@ int tp3d_oc_update(int nelx, int nely, int nelz, double rmin, const double* x,
  * tp3d_oc_noalloc_max_elements() (262144) elements are rejected with
  * TP3D_ERR_ARG.  The first call on a device looks up the array's address
  * (cudaGetSymbolAddress) and should come before any stream capture.  Each
- * call queues only device work on `stream` (the filter column table is built
- * in the array by a small kernel, the barrier words and stats are cleared by
- * memsets): no host buffer is read after the call returns.  All calls share
+ * call queues only device work on `stream` (the barrier words and stats are
+ * cleared by memsets): no host buffer is read after the call returns.  All calls share
  * the array, so calls that overlap on the GPU race; issue them on one stream.
  * Arguments and results are those of tp3d_oc_update. */
 long long tp3d_oc_noalloc_max_elements(void);
@@ -229,8 +228,9 @@ typedef struct tp3d_solver_opts {
                            little and saves CG iterations (measured on the 128x64x64 cantilever) */
   int pdl;              /* programmatic dependent launch in the CG loop (each kernel's launch overlaps
                            the tail of the one before it), a mask: 1 the coarse levels' kernels,
-                           2 the fine operator and fine-level vector kernels, 3 both, 0 plain stream
-                           order.  Turned off by itself when a CUDA graph cannot be built with it. */
+                           2 the fine operator, the fine-level vector kernels and the kernels of the
+                           FP64 cycle's small levels (at most split_dofs DOFs), 3 both, 0 plain
+                           stream order.  Turned off by itself when a CUDA graph cannot be built with it. */
   int coarse_bf16;      /* mixed form: levels 1 .. coarse_bf16 (default 99: every level but the
                            dense coarsest) store their packed stencils in bf16 (symmetrized, FP32
                            arithmetic), halving the bytes each smoothing step there reads; 0 all

@@ -786,9 +786,9 @@ struct tp3d_solver {
   // The programmatic-launch class of the kernels over level L: the fine operator's
   // class for the fine level and for the FP64 cycle's small levels, whose kernels
   // last little longer than a launch (32x16x16 loop bodies 10.95 to 10.5 ms, 48x24x24
-  // gradient 16.1 to 15.5).  On
-  // the larger coarse levels the early blocks cost more than they save (128x64x64
-  // FP64 +3%), and so they do on the mixed form's levels (61x30x37 +2%).
+  // gradient 16.1 to 15.5).  On the larger coarse levels the early blocks cost more
+  // than they save (128x64x64 FP64 +3%), and so they do on the mixed form's levels
+  // (61x30x37 +2%).
   template <typename T>
   int pdl_class(int L) const {
     return L == 0 || (sizeof(T) == 8 && 3 * grids[L].nnode() <= o.split_dofs) ? kPdlFine : kPdlCoarse;
