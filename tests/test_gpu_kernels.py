@@ -365,3 +365,37 @@ def test_oc_walk_matches_oracle_path(P, dims, rmin, spread, frac):
     # the same multiplier: candidates to rounding, filtered densities to the filter's 1e-12
     np.testing.assert_allclose(from_flat(xn, shape).cpu().numpy(), xo, rtol=0, atol=1e-14)
     np.testing.assert_allclose(from_flat(rn, shape).cpu().numpy(), rhoo, rtol=0, atol=1e-12)
+
+
+# Boolean device masks are read in place: every layout and type of mask that the
+# calls take gives the numpy masks' result bit for bit, and the mask stays as it was.
+@pytest.mark.parametrize("form", ["bool_c", "bool_fortran", "bool_strided", "uint8", "int64"])
+def test_device_masks_match_numpy_masks(P, form):
+    rng = np.random.default_rng(4)
+    shape = (9, 33, 5)
+    x, g = rng.uniform(0.2, 0.9, size=shape), -rng.uniform(0.1, 1.0, size=shape)
+    solid = rng.uniform(size=shape) < 0.2
+    void = (rng.uniform(size=shape) < 0.2) & ~solid
+
+    def dev(m):
+        t = torch.as_tensor(m).cuda()
+        if form == "bool_fortran":
+            return t.permute(2, 1, 0).contiguous().permute(2, 1, 0)
+        if form == "bool_strided":
+            return torch.stack([t, ~t], dim=3)[..., 0]
+        return t if form == "bool_c" else t.to(getattr(torch, form))
+
+    H, Hs = P.build_filter(33, 9, 5, 2.3)
+    want = P.build_physical_density(x, H, Hs, 2.0, 0.5, solid, void)
+    s, v, f = dev(solid), dev(void), dev(~(solid | void))
+    got = P.build_physical_density(torch.as_tensor(x).cuda(), H, Hs, 2.0, 0.5, s, v)
+    for a, b in zip(got, want):
+        np.testing.assert_array_equal(a.cpu().numpy(), b)
+    dv = P.apply_density_filter_chain_rule((~(solid | void)).astype(float), want[2], H, Hs)
+    target = 0.8 * want[1][~(solid | void)].sum()
+    wx, wr = P.optimality_criteria_update_projected(x, g, dv, 0.2, target, H, Hs, 2.0, 0.5, ~(solid | void), solid, void)
+    gx, gr = P.optimality_criteria_update_projected(*(torch.as_tensor(a).cuda() for a in (x, g, dv)), 0.2, target, H, Hs,
+                                                    2.0, 0.5, f, s, v)
+    np.testing.assert_array_equal(gx.cpu().numpy(), wx)
+    np.testing.assert_array_equal(gr.cpu().numpy(), wr)
+    np.testing.assert_array_equal(s.bool().cpu().numpy(), solid)
