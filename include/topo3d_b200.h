@@ -122,8 +122,9 @@ int tp3d_oc_update(int nelx, int nely, int nelz, double rmin, const double* x,
  * tp3d_oc_noalloc_max_elements() (262144) elements are rejected with
  * TP3D_ERR_ARG.  The first call on a device looks up the array's address
  * (cudaGetSymbolAddress) and should come before any stream capture.  Each
- * call queues only device work on `stream` (the barrier words and stats are
- * cleared by memsets): no host buffer is read after the call returns.  All calls share
+ * call queues only device work on `stream` (the filter column table is built
+ * in the array by a small kernel, the barrier words and stats are cleared by
+ * memsets): no host buffer is read after the call returns.  All calls share
  * the array, so calls that overlap on the GPU race; issue them on one stream.
  * Arguments and results are those of tp3d_oc_update. */
 long long tp3d_oc_noalloc_max_elements(void);

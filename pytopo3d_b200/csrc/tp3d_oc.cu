@@ -4,12 +4,12 @@
 //
 // The reference re-filters and re-projects a candidate design for every
 // bisection step and syncs the volume to the host.  Here the whole loop runs
-// in one persistent kernel: every block owns filter tiles, marches the
-// candidate x(lambda) of its tiles (+ halo) through the filter, projects and
-// sums the free volume; per-block partials are combined in a fixed order after
-// a (bounded) grid barrier, so every block takes the same decision.  Only the
-// best multiplier is kept; the best candidate is recomputed from it at the
-// end, so no candidate array is stored.
+// in one persistent kernel: every block owns a set of filter tiles, stages the
+// candidate x(lambda) of its tiles (+ halo) in shared memory, filters,
+// projects and sums the free volume; per-block partials are combined in a
+// fixed order after a (bounded) grid barrier, so every block takes the same
+// bisection decision.  Only the best multiplier is kept; the best candidate is
+// recomputed from it at the end, so no candidate array is stored.
 //
 // An evaluation costs a pass over the design and a grid barrier, so the kernel
 // makes few of them: the reference's bisection path (about 65 steps) is
@@ -27,10 +27,11 @@ namespace tp3d {
 namespace {
 
 constexpr int kOcMaxBlocks = 4096;
+constexpr int kOcBatch = 8;  // staged candidates per thread whose loads are in flight together
 
 struct OcArgs {
   Grid g;
-  FilterTiles tiles;
+  FilterCols fc;
   const double* x;
   const double* dc;
   const double* dv;
@@ -77,58 +78,55 @@ __device__ __forceinline__ double candidate_q(double xe, double q, double isl, d
   return fmin(fmax(c, 0.0), 1.0);
 }
 
-// The candidate at a multiplier as the filter's input (arrays written earlier in
-// this launch are read through L2, __ldcg, never the L1 path).
-struct OcSrc {
-  const double *x, *ratio;
-  double isl, move;
-  bool keep;  // no multiplier was found: the design itself
-  struct Raw {
-    double x, q;
-  };
-  __device__ Raw load(long long pz, unsigned i) const { return {__ldg(x + pz + i), __ldcg(ratio + pz + i)}; }
-  __device__ double value(const Raw& r) const { return keep ? r.x : candidate_q(r.x, r.q, isl, move); }
-};
-struct OcOutVolume {
-  const double *Hs, *ratio;
-  const Projection& pr;
-  double sum;
-  struct Pre {
-    double Hs, q;
-  };
-  __device__ Pre load(long long pz, unsigned i) const { return {__ldg(Hs + pz + i), __ldcg(ratio + pz + i)}; }
-  __device__ void store(long long, unsigned, const Pre& p, double v) {
-    if (p.q >= 0.0) sum += pr.value(v / p.Hs, nullptr);
-  }
-};
-struct OcOutDensity {
-  const double *Hs, *ratio;
-  const Projection& pr;
-  double* rho;
-  struct Pre {
-    double Hs, q;
-  };
-  __device__ Pre load(long long pz, unsigned i) const { return {__ldg(Hs + pz + i), __ldcg(ratio + pz + i)}; }
-  __device__ void store(long long pz, unsigned i, const Pre& p, double v) const {
-    double r = pr.value(v / p.Hs, nullptr);
-    if (p.q == kCodeSolid) r = 1.0;
-    if (p.q == kCodeVoid) r = 0.0;
-    (rho + pz)[i] = r;
-  }
-};
-
 // Projected free volume of the candidate at multiplier lam (oc_update.py:78-111):
-// march the candidate of each owned tile through the filter, project, sum;
-// per-block partials go to `part`, and after the grid barrier every block sums
-// them in the same order.  Returns false if the barrier wait expired.
+// stage candidates of each owned tile (+ halo), filter, project, sum; per-block
+// partials go to `part`, and after the grid barrier every block sums them in the
+// same order.  Returns false if the barrier wait expired.  (Arrays written
+// earlier in this launch are read through L2, __ldcg, never the L1 path.)
 template <int Z>
-__device__ __noinline__ bool oc_volume(const OcArgs& a, const RingWeights<Z>& W, double lam, double* part, double* s,
-                                       double* red, double* vol) {
-  const OcSrc src{a.x, a.ratio, 1.0 / sqrt(lam + 1e-30), a.move, false};
-  OcOutVolume out{a.Hs, a.ratio, a.pr, 0.0};
-  const long long ntiles = a.tiles.count();
-  for (long long t = blockIdx.x; t < ntiles; t += gridDim.x) filter_march<Z>(a.g, W, a.tiles, t, s, src, out);
-  const double vpart = block_sum(out.sum, red);
+__device__ bool oc_volume(const OcArgs& a, double lam, double* part, double* s, double* red, double* vol) {
+  constexpr int SY = kFilterTY + 2 * Z, SX = kFilterTX + 2 * Z, SZ = kFilterKZ + 2 * Z;
+  constexpr int NS = SY * SX * SZ;
+  const long long ntiles = filter_ntiles(a.g);
+  const double isl = 1.0 / sqrt(lam + 1e-30);
+  double vpart = 0.0;
+  for (long long t = blockIdx.x; t < ntiles; t += gridDim.x) {
+    const FilterTile tile = filter_tile_at(a.g, t);
+    __syncthreads();
+    // kOcBatch elements per thread at a time: all their loads are issued
+    // before the first candidate is formed, so they are in flight together
+    for (int i0 = threadIdx.x; i0 < NS; i0 += kOcBatch * kFilterThreads) {
+      double xv[kOcBatch], qv[kOcBatch];
+      unsigned in = 0;
+#pragma unroll
+      for (int b = 0; b < kOcBatch; ++b) {
+        const int i = i0 + b * kFilterThreads;
+        xv[b] = 0.0;
+        qv[b] = 0.0;
+        if (i < NS) {
+          const int ly = i % SY, r = i / SY;
+          const int lx = r % SX, lz = r / SX;
+          const int gx = tile.x0 + lx - Z, gy = tile.y0 + ly - Z, gz = tile.z0 + lz - Z;
+          if (gx >= 0 && gx < a.g.nx && gy >= 0 && gy < a.g.ny && gz >= 0 && gz < a.g.nz) {
+            const long long e = a.g.eidx(gx, gy, gz);
+            xv[b] = __ldg(&a.x[e]);
+            qv[b] = __ldcg(&a.ratio[e]);
+            in |= 1u << b;
+          }
+        }
+      }
+#pragma unroll
+      for (int b = 0; b < kOcBatch; ++b) {
+        const int i = i0 + b * kFilterThreads;
+        if (i < NS) s[i] = ((in >> b) & 1u) ? candidate_q(xv[b], qv[b], isl, a.move) : 0.0;
+      }
+    }
+    __syncthreads();
+    filter_apply<Z>(a.g, a.fc, tile, s, [&](long long e, int, int, int, double v) {
+      if (__ldcg(&a.ratio[e]) >= 0.0) vpart += a.pr.value(v / __ldg(&a.Hs[e]), nullptr);
+    });
+  }
+  vpart = block_sum(vpart, red);
   if (threadIdx.x == 0) part[blockIdx.x] = vpart;
   if (!grid_sync_flip(a.bar.count, a.bar.err, a.spin_limit, a.phantom)) return false;
   *vol = sum_partials(part, gridDim.x, red);
@@ -145,10 +143,11 @@ __device__ __forceinline__ bool bisection_done(double lo, double hi, double tol)
 }
 
 template <int Z>
-__global__ void __launch_bounds__(kFilterThreads, filter_blocks_per_sm(Z)) oc_kernel(const __grid_constant__ OcArgs a,
-                                                            const __grid_constant__ RingWeights<Z> W) {
-  __shared__ __align__(16) double s[2 * filter_plane(Z)];
+__global__ void __launch_bounds__(kFilterThreads) oc_kernel(const __grid_constant__ OcArgs a) {
+  extern __shared__ double s[];
+  filter_cols_to_smem<Z>(a.fc, s);  // read back after the first barrier
   __shared__ double red[32];
+  const long long ntiles = filter_ntiles(a.g);
   const long long nele = a.g.nele();
   const int nblk = gridDim.x;
   auto solid_at = [&](long long e) { return a.solid && a.solid[e]; };
@@ -206,14 +205,14 @@ __global__ void __launch_bounds__(kFilterThreads, filter_blocks_per_sm(Z)) oc_ke
   // go to the ordinary steps below instead.
   // About 10 evaluations in place of the path's 72 to 78 (of which a search over
   // the halvings by bisection and one evaluation per later step took 34):
-  // 828 us before and 310 now at 128x64x64, rmin 3; 13.0 and 3.0 ms at
-  // 256x128x128, rmin 4.5; 618 and 165 us at 32x16x16.
+  // 828 us before and 330 now at 128x64x64, rmin 3; 13.0 and 4.4 ms at
+  // 256x128x128, rmin 4.5; 618 and 207 us at 32x16x16.
   double lo = 0.0, hi = 1.0e12;
   double best_err = INFINITY, best_lam = NAN, best_vol = NAN;
   int it = 0, pass = 0;
   bool done = false;
   auto eval = [&](double lam, double* v) {
-    return oc_volume<Z>(a, W, lam, (pass++ & 1) ? a.partB : a.partA, s, red, v);
+    return oc_volume<Z>(a, lam, (pass++ & 1) ? a.partB : a.partA, s, red, v);
   };
   auto record = [&](double lam, double vol) {
     const double err = fabs(vol - a.target);
@@ -399,19 +398,32 @@ __global__ void __launch_bounds__(kFilterThreads, filter_blocks_per_sm(Z)) oc_ke
 
   // ---- best candidate, its density, and change (optimizer.py:642) ----
   const bool have = !isnan(best_lam);
-  const OcSrc src{a.x, a.ratio, have ? 1.0 / sqrt(best_lam + 1e-30) : 0.0, a.move, !have};
+  const double isl = have ? 1.0 / sqrt(best_lam + 1e-30) : 0.0;
+  auto best = [&](long long e) {
+    const double xe = __ldg(&a.x[e]);
+    return have ? candidate_q(xe, __ldcg(&a.ratio[e]), isl, a.move) : xe;
+  };
   double cmax = 0.0;
   for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < nele; e += (long long)nblk * blockDim.x) {
-    const OcSrc::Raw r = src.load(e, 0);
-    const double v = src.value(r);
+    const double xe = __ldg(&a.x[e]), v = best(e);
     a.x_new[e] = v;
-    if (r.q >= 0.0) cmax = fmax(cmax, fabs(v - r.x));
+    if (a.ratio[e] >= 0.0) cmax = fmax(cmax, fabs(v - xe));
   }
   cmax = block_max(cmax, red);
   if (threadIdx.x == 0) a.partC[blockIdx.x] = cmax;
-  OcOutDensity out{a.Hs, a.ratio, a.pr, a.rho_new};
-  const long long ntiles = a.tiles.count();
-  for (long long t = blockIdx.x; t < ntiles; t += nblk) filter_march<Z>(a.g, W, a.tiles, t, s, src, out);
+  for (long long t = blockIdx.x; t < ntiles; t += nblk) {
+    const FilterTile tile = filter_tile_at(a.g, t);
+    __syncthreads();
+    filter_stage<Z>(a.g, tile, s, [&](long long e, int, int, int) { return best(e); });
+    __syncthreads();
+    filter_apply<Z>(a.g, a.fc, tile, s, [&](long long e, int, int, int, double v) {
+      double r = a.pr.value(v / __ldg(&a.Hs[e]), nullptr);
+      const double q = __ldcg(&a.ratio[e]);
+      if (q == kCodeSolid) r = 1.0;
+      if (q == kCodeVoid) r = 0.0;
+      a.rho_new[e] = r;
+    });
+  }
   if (!grid_sync_flip(a.bar.count, a.bar.err, a.spin_limit, a.phantom)) return;
   if (blockIdx.x == 0) {
     double t = 0.0;
@@ -430,25 +442,23 @@ __global__ void __launch_bounds__(kFilterThreads, filter_blocks_per_sm(Z)) oc_ke
   }
 }
 
-// The cooperative launch: as many blocks as are co-resident, the tiles split for them.
+// The cooperative launch: as many blocks as are co-resident, a tile each or more.
 template <int Z>
-int oc_launch(OcArgs a, double rmin, cudaStream_t st) {
+int oc_launch(OcArgs a, cudaStream_t st) {
   auto kern = oc_kernel<Z>;
+  const size_t smem = filter_smem_bytes(Z);
+  if (int rc = ensure_dynamic_smem(kern, smem)) return rc;
   int dev = 0, nsm = 0, per_sm = 0;
   TP3D_CHECK(cudaGetDevice(&dev));
   TP3D_CHECK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-  TP3D_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kFilterThreads, 0));
+  TP3D_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kFilterThreads, smem));
   if (per_sm < 1) {
     tp3d_set_last_error("OC kernel does not fit on an SM");
     return TP3D_ERR_CUDA;
   }
-  const long long slots = std::min<long long>((long long)per_sm * nsm, kOcMaxBlocks);
-  a.tiles = filter_tiles(a.g, Z, nsm, slots);
-  RingWeights<Z> W = ring_weights<Z>(rmin);
-  void* args[] = {&a, &W};
-  TP3D_CHECK(cudaLaunchCooperativeKernel((const void*)kern, dim3((unsigned)std::min(slots, a.tiles.count())),
-                                         dim3(kFilterThreads), args, 0, st));
-  add_launches(1);
+  const long long grid = std::min({(long long)per_sm * nsm, filter_ntiles(a.g), (long long)kOcMaxBlocks});
+  void* args[] = {&a};
+  TP3D_CHECK(cudaLaunchCooperativeKernel((const void*)kern, dim3((unsigned)grid), dim3(kFilterThreads), args, smem, st));
   return TP3D_OK;
 }
 
@@ -483,13 +493,13 @@ extern "C" int tp3d_oc_update(int nelx, int nely, int nelz, double rmin, const d
     tp3d_set_last_error("invalid projection parameters");
     return TP3D_ERR_ARG;
   }
-  int Z = 0;
-  if (int rc = filter_z_for(rmin, &Z)) return rc;
+  FilterCols fc;
+  if (int rc = filter_cols_for(rmin, &fc)) return rc;
   const Grid g{nelx, nely, nelz};
   const long long n = g.nele();
   cudaStream_t st = (cudaStream_t)stream;
 
-  OcArgs a{g, FilterTiles{}, x, dc_dx, dv_dx, Hs, solid, void_, move, target_free_volume, bisection_tol,
+  OcArgs a{g, fc, x, dc_dx, dv_dx, Hs, solid, void_, move, target_free_volume, bisection_tol,
            max_bisection, Projection(beta, eta), x_new, rho_new, stats};
   set_wait_policy(a);
   double* base = (double*)scratch;
@@ -505,7 +515,8 @@ extern "C" int tp3d_oc_update(int nelx, int nely, int nelz, double rmin, const d
   // NaN stats mark a launch that did not finish (e.g. an expired barrier wait)
   TP3D_CHECK(cudaMemsetAsync(stats, 0xff, 8 * sizeof(double), st));
 
-  TP3D_DISPATCH_Z(Z, return oc_launch<ZC>(a, rmin, st));
+  TP3D_DISPATCH_Z(fc.Z, if (int rc = oc_launch<ZC>(a, st)) return rc);
+  add_launches(1);
   return TP3D_OK;
 }
 
@@ -516,17 +527,21 @@ extern "C" int tp3d_oc_update(int nelx, int nely, int nelz, double rmin, const d
 // whose device memory is fully reserved up front by its own allocator, or code
 // that cannot accept the implicit device synchronisation that cudaMalloc /
 // cudaFree bring.  The scratch of the bisection (normalised ratios, per-block
-// partial sums, barrier counters) lives in one
+// partial sums, barrier counters, filter column table) lives in one
 // file-scope __device__ array instead.  Every GPU that loads this library
 // holds that array (about 2.2 MB) until the process exits.
 // ---------------------------------------------------------------------------
 namespace tp3d_oc_noalloc {
 
 constexpr long long kNoAllocMaxElements = 1LL << 18;  // e.g. 64x64x64 or 128x64x32
+constexpr int kNoAllocMaxCols = (2 * kFilterMaxZ + 1) * (2 * kFilterMaxZ + 1);
 constexpr size_t kNoAllocRatioBytes = (size_t)kNoAllocMaxElements * sizeof(double);
 constexpr size_t kNoAllocPartBytes = (size_t)3 * kOcMaxBlocks * sizeof(double);
 constexpr size_t kNoAllocBarrierBytes = 256;
-constexpr size_t kNoAllocBytes = kNoAllocRatioBytes + kNoAllocPartBytes + kNoAllocBarrierBytes;
+constexpr size_t kNoAllocDxyBytes = ((kNoAllocMaxCols * sizeof(int2) + 255) / 256) * 256;
+constexpr size_t kNoAllocWBytes = (size_t)kNoAllocMaxCols * (2 * kFilterMaxZ + 1) * sizeof(double);
+constexpr size_t kNoAllocBytes =
+    kNoAllocRatioBytes + kNoAllocPartBytes + kNoAllocBarrierBytes + kNoAllocDxyBytes + kNoAllocWBytes;
 
 static __device__ __align__(256) unsigned char g_oc_noalloc_scratch[kNoAllocBytes];
 
@@ -555,6 +570,26 @@ int noalloc_scratch(void** out) {
   *out = g_noalloc_addr[dev];
   return TP3D_OK;
 }
+
+// The filter column table of a radius, built in place in the static scratch:
+// thread i evaluates candidate column i (filter_column, the same function and
+// order as the host-built tables of the allocating path) and writes it at its
+// rank among the columns that have a tap.  No host buffer is involved.
+__global__ void __launch_bounds__(256) noalloc_columns_kernel(double rmin, int Z, int2* dxy, double* w) {
+  __shared__ int has_tap[256];
+  const int W = 2 * Z + 1, i = threadIdx.x;
+  double col[2 * kFilterMaxZ + 1];
+  const bool any = i < W * W && filter_column(rmin, Z, i, col);
+  has_tap[i] = any ? 1 : 0;
+  __syncthreads();
+  if (any) {
+    int pos = 0;
+    for (int k = 0; k < i; ++k) pos += has_tap[k];
+    dxy[pos] = make_int2(i / W - Z, i % W - Z);
+    for (int j = 0; j < W; ++j) w[(size_t)pos * W + j] = col[j];
+  }
+}
+static_assert((2 * kFilterMaxZ + 1) * (2 * kFilterMaxZ + 1) <= 256, "one thread per candidate column");
 
 }  // namespace tp3d_oc_noalloc
 using namespace tp3d_oc_noalloc;
@@ -588,15 +623,19 @@ extern "C" int tp3d_oc_update_noalloc(int nelx, int nely, int nelz, double rmin,
     tp3d_set_last_error("invalid projection parameters");
     return TP3D_ERR_ARG;
   }
-  int Z = 0;
-  if (int rc = filter_z_for(rmin, &Z)) return rc;
+  const int Z = filter_radius_z(rmin);
+  if (Z < 0 || !std::isfinite(rmin)) return TP3D_ERR_ARG;
+  if (Z > kFilterMaxZ) {
+    tp3d_set_last_error("rmin too large for the stencil filter (max 7)");
+    return TP3D_ERR_ARG;
+  }
   void* base_v = nullptr;
   if (int rc = noalloc_scratch(&base_v)) return rc;
   unsigned char* base = (unsigned char*)base_v;
   cudaStream_t st = (cudaStream_t)stream;
 
   const Grid g{nelx, nely, nelz};
-  OcArgs a{g, FilterTiles{}, x, dc_dx, dv_dx, Hs, solid, void_, move, target_free_volume, bisection_tol,
+  OcArgs a{g, FilterCols{}, x, dc_dx, dv_dx, Hs, solid, void_, move, target_free_volume, bisection_tol,
            max_bisection, Projection(beta, eta), x_new, rho_new, stats};
   set_wait_policy(a);
   a.ratio = (double*)base;
@@ -607,11 +646,21 @@ extern "C" int tp3d_oc_update_noalloc(int nelx, int nely, int nelz, double rmin,
   a.bar.count = bar;
   a.bar.gen = bar + 1;
   a.bar.err = (int*)(bar + 2);
-  // The array keeps the previous call's contents: the barrier counters are cleared on every call.
+  int2* d_dxy = (int2*)(base + kNoAllocRatioBytes + kNoAllocPartBytes + kNoAllocBarrierBytes);
+  double* d_w = (double*)((unsigned char*)d_dxy + kNoAllocDxyBytes);
+  a.fc.dxy = d_dxy;
+  a.fc.w = d_w;
+  a.fc.ncols = filter_columns_build(rmin, Z, nullptr, nullptr);  // count only
+  a.fc.Z = Z;
+  // The array keeps the previous call's contents: the column table is
+  // rebuilt on the device and the barrier counters cleared on every call.
+  noalloc_columns_kernel<<<1, 256, 0, st>>>(rmin, Z, d_dxy, d_w);
+  TP3D_CHECK_LAUNCH();
   TP3D_CHECK(cudaMemsetAsync(bar, 0, kNoAllocBarrierBytes, st));
   TP3D_CHECK(cudaMemsetAsync(stats, 0xff, 8 * sizeof(double), st));
 
-  TP3D_DISPATCH_Z(Z, return oc_launch<ZC>(a, rmin, st));
+  TP3D_DISPATCH_Z(Z, if (int rc = oc_launch<ZC>(a, st)) return rc);
+  add_launches(2);
   return TP3D_OK;
 }
 

@@ -1,6 +1,9 @@
 """CUDA filter / projection / chain-rule / element-energy / OC kernels against the oracle
 and the reference's golden vectors (FP64, tolerance 1e-12 unless stated)."""
 
+import math
+from fractions import Fraction
+
 import numpy as np
 import pytest
 import torch
@@ -50,6 +53,35 @@ def test_filter_projection_and_transpose_match_oracle(P, g):
         out = P.apply_density_filter_chain_rule(gph, dp, H, Hs)
         np.testing.assert_allclose(out, O.apply_density_filter_chain_rule(gph, dpo, Ho, Hso), rtol=1e-12,
                                    atol=1e-13 * np.abs(gph).max())
+
+
+def _fma(a, b, c):
+    return float(Fraction(a) * Fraction(b) + Fraction(c))
+
+
+# The FP64 loop amplifies the rounding of the filtered densities (a change of one
+# unit in the last place of the design moves its results by up to 5e-8 where the
+# solve ends at its residual floor), so the filter's sums keep their order to the
+# bit: one fused multiply-add per tap, columns (dx, dy) in row-major order, dz
+# ascending within a column.
+@pytest.mark.parametrize("dims,rmin", [((5, 4, 9), 2.5), ((3, 33, 2), 1.5), ((9, 3, 8), 3.0), ((4, 5, 3), 4.4)])
+def test_filter_sums_keep_their_order(P, dims, rmin):
+    nx, ny, nz = dims
+    x = np.random.default_rng(nx).uniform(size=(ny, nx, nz))
+    r = range(-int(rmin), int(rmin) + 1)
+    taps = [(dx, dy, dz, rmin - math.sqrt(dx * dx + dy * dy + dz * dz)) for dx in r for dy in r for dz in r]
+    want, sums = np.empty_like(x), np.empty_like(x)
+    for iy, ix, iz in np.ndindex(x.shape):
+        v = h = 0.0
+        for dx, dy, dz, w in taps:
+            if w > 1e-9 and 0 <= ix + dx < nx and 0 <= iy + dy < ny and 0 <= iz + dz < nz:
+                v = _fma(w, x[iy + dy, ix + dx, iz + dz], v)
+                h = h + w
+        want[iy, ix, iz], sums[iy, ix, iz] = v / h, h
+    H, Hs = P.build_filter(nx, ny, nz, rmin)
+    np.testing.assert_array_equal(Hs.cpu().numpy(), sums.transpose(2, 1, 0).reshape(-1))
+    rf, _, _ = P.build_physical_density(x, H, Hs, 2.0, 0.5, np.zeros_like(x, bool), np.zeros_like(x, bool))
+    np.testing.assert_array_equal(rf, want)
 
 
 def test_projection_matches_golden(P, golden):
