@@ -103,7 +103,9 @@ int tp3d_sensitivity(int nelx, int nely, int nelz, double rmin, const double* U,
  * stats (device, 8 doubles): [lambda_best, volume_best, steps, change,
  *   ratio_scale, lambda_lo, lambda_hi, best_error].
  * change = max |x_new - x| over free elements (optimizer.py:642).
- * `scratch` holds >= tp3d_oc_scratch_bytes() bytes of device memory. */
+ * `scratch` holds >= tp3d_oc_scratch_bytes() bytes of device memory.
+ * x_new or rho_new may be x itself (an update in place); otherwise the outputs
+ * overlap neither the inputs nor each other. */
 size_t tp3d_oc_scratch_bytes(int nelx, int nely, int nelz, double rmin);
 int tp3d_oc_update(int nelx, int nely, int nelz, double rmin, const double* x,
                    const double* dc_dx, const double* dv_dx, const double* Hs,

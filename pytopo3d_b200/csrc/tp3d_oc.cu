@@ -399,22 +399,21 @@ __global__ void __launch_bounds__(kFilterThreads) oc_kernel(const __grid_constan
   // ---- best candidate, its density, and change (optimizer.py:642) ----
   const bool have = !isnan(best_lam);
   const double isl = have ? 1.0 / sqrt(best_lam + 1e-30) : 0.0;
-  auto best = [&](long long e) {
-    const double xe = __ldg(&a.x[e]);
-    return have ? candidate_q(xe, __ldcg(&a.ratio[e]), isl, a.move) : xe;
-  };
   double cmax = 0.0;
   for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < nele; e += (long long)nblk * blockDim.x) {
-    const double xe = __ldg(&a.x[e]), v = best(e);
+    const double xe = __ldg(&a.x[e]), q = a.ratio[e];
+    const double v = have ? candidate_q(xe, q, isl, a.move) : xe;
     a.x_new[e] = v;
-    if (a.ratio[e] >= 0.0) cmax = fmax(cmax, fabs(v - xe));
+    if (q >= 0.0) cmax = fmax(cmax, fabs(v - xe));
   }
   cmax = block_max(cmax, red);
   if (threadIdx.x == 0) a.partC[blockIdx.x] = cmax;
+  // x is not read after this barrier: x_new or rho_new may be x
+  if (!grid_sync_flip(a.bar.count, a.bar.err, a.spin_limit, a.phantom)) return;
   for (long long t = blockIdx.x; t < ntiles; t += nblk) {
     const FilterTile tile = filter_tile_at(a.g, t);
     __syncthreads();
-    filter_stage<Z>(a.g, tile, s, [&](long long e, int, int, int) { return best(e); });
+    filter_stage<Z>(a.g, tile, s, [&](long long e, int, int, int) { return __ldcg(&a.x_new[e]); });
     __syncthreads();
     filter_apply<Z>(a.g, a.fc, tile, s, [&](long long e, int, int, int, double v) {
       double r = a.pr.value(v / __ldg(&a.Hs[e]), nullptr);
@@ -424,7 +423,6 @@ __global__ void __launch_bounds__(kFilterThreads) oc_kernel(const __grid_constan
       a.rho_new[e] = r;
     });
   }
-  if (!grid_sync_flip(a.bar.count, a.bar.err, a.spin_limit, a.phantom)) return;
   if (blockIdx.x == 0) {
     double t = 0.0;
     for (int i = threadIdx.x; i < nblk; i += blockDim.x) t = fmax(t, __ldcg(&a.partC[i]));

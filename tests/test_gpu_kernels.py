@@ -399,6 +399,41 @@ def test_oc_walk_matches_oracle_path(P, dims, rmin, spread, frac):
     np.testing.assert_allclose(from_flat(rn, shape).cpu().numpy(), rhoo, rtol=0, atol=1e-12)
 
 
+# An update in place: the new design or its density over the old design, on a grid
+# of several tiles in every direction, gives what separate outputs give.
+@pytest.mark.parametrize("out", ["x_new", "rho_new"])
+@pytest.mark.parametrize("noalloc", [False, True])
+def test_oc_update_in_place(P, out, noalloc):
+    from pytopo3d_b200 import _lib
+    from pytopo3d_b200._tensors import to_flat, vec
+
+    L = _lib.lib()
+    nx, ny, nz, rmin = 24, 70, 20, 2.5
+    rng = np.random.default_rng(6)
+    x = to_flat(rng.uniform(0.1, 0.9, size=(ny, nx, nz)))
+    dc, dv = -torch.exp(to_flat(rng.normal(size=(ny, nx, nz)))), torch.ones_like(x)
+    _, Hs = P.build_filter(nx, ny, nz, rmin)
+    Hs = vec(Hs)
+    scratch = torch.empty(L.tp3d_oc_scratch_bytes(nx, ny, nz, rmin), dtype=torch.uint8, device="cuda")
+
+    def run(x, x_new, rho_new):
+        stats = torch.empty(8, dtype=torch.float64, device="cuda")
+        args = [nx, ny, nz, rmin, x.data_ptr(), dc.data_ptr(), dv.data_ptr(), Hs.data_ptr(), None, None, 0.2,
+                0.4 * x.numel(), 2.0, 0.5, 80, 1e-8, x_new.data_ptr(), rho_new.data_ptr(), stats.data_ptr()]
+        if noalloc:
+            _lib.check(L.tp3d_oc_update_noalloc(*args, _lib.stream_ptr()), "oc")
+        else:
+            _lib.check(L.tp3d_oc_update(*args, scratch.data_ptr(), _lib.stream_ptr()), "oc")
+        return x_new, rho_new, stats
+
+    want = run(x, torch.empty_like(x), torch.empty_like(x))
+    for _ in range(5):
+        y = x.clone()
+        got = run(y, *((y, torch.empty_like(x)) if out == "x_new" else (torch.empty_like(x), y)))
+        for a, b in zip(got, want):
+            assert torch.equal(a, b)
+
+
 # Boolean device masks are read in place: every layout and type of mask that the
 # calls take gives the numpy masks' result bit for bit, and the mask stays as it was.
 @pytest.mark.parametrize("form", ["bool_c", "bool_fortran", "bool_strided", "uint8", "int64"])
