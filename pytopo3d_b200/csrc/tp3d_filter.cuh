@@ -16,7 +16,8 @@
 // later by more than 2e-9 on 6 of 40 random grids with protected voids.  Ring sums
 // per plane marched along z round differently and were taken back for that: filter
 // and projection 17 us at 128x64x64 (rmin 3) and 169 us at 256x128x128 (rmin 4.5)
-// against 23 and 294 us here, OC update 385 and 3091 us against 330 and 4446.
+// against 23 and 294 us here, OC update (the same evaluations) 385 and 3091 us
+// against 330 and 4446.
 #pragma once
 
 #include "tp3d_common.cuh"

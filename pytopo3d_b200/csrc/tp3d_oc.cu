@@ -202,11 +202,12 @@ __global__ void __launch_bounds__(kFilterThreads) oc_kernel(const __grid_constan
   // step with the smallest error (strict <, oc_update.py:106).  Equal volumes at
   // two multipliers (a plateau, e.g. every candidate held at its move limit),
   // volumes that are not finite, and searches that reach an end of the halvings
-  // go to the ordinary steps below instead.
-  // About 10 evaluations in place of the path's 72 to 78 (of which a search over
+  // go to the ordinary steps below instead.  (The path's end before the chosen one
+  // is evaluated for this alone: a plateau may lie between two evaluations.)
+  // About 11 evaluations in place of the path's 72 to 78 (of which a search over
   // the halvings by bisection and one evaluation per later step took 34):
-  // 828 us before and 330 now at 128x64x64, rmin 3; 13.0 and 4.4 ms at
-  // 256x128x128, rmin 4.5; 618 and 207 us at 32x16x16.
+  // 828 us before and 349 now at 128x64x64, rmin 3; 13.0 and 4.7 ms at
+  // 256x128x128, rmin 4.5; 618 and 228 us at 32x16x16.
   double lo = 0.0, hi = 1.0e12;
   double best_err = INFINITY, best_lam = NAN, best_vol = NAN;
   int it = 0, pass = 0;
@@ -261,10 +262,11 @@ __global__ void __launch_bounds__(kFilterThreads) oc_kernel(const __grid_constan
     double A = ldexp(1.0e12, -jhi), VA = vhi, B = ldexp(1.0e12, -jlo), VB = vlo;
     double t0 = 1.0 / sqrt(A), v0 = VA, t1 = 1.0 / sqrt(B), v1 = VB;
     double wlo = 0.0, whi = 1.0e12, width = B - A;  // the walk's own state
-    int wit = 0, ilo = -1, ihi = -1, slow = 0;       // ilo, ihi: steps that set its ends
+    double plo = 0.0, phi = 1.0e12;                  // its ends before the last ones
+    int wit = 0, slow = 0;
     __shared__ struct {
-      double lo, hi, e;
-      int it, ilo, ihi, done;
+      double lo, hi, plo, phi, e;
+      int it, done;
     } w;
     while (walk) {
       // one warp walks and picks the next multiplier: the steps are a chain of
@@ -273,8 +275,8 @@ __global__ void __launch_bounds__(kFilterThreads) oc_kernel(const __grid_constan
         bool wdone = false;
         while (!wdone && wit < a.max_iter) {
           const double mid = 0.5 * (wlo + whi);
-          if (mid <= A) wlo = mid, ilo = wit;
-          else if (mid >= B) whi = mid, ihi = wit;
+          if (mid <= A) plo = wlo, wlo = mid;
+          else if (mid >= B) phi = whi, whi = mid;
           else break;
           ++wit;
           wdone = bisection_done(wlo, whi, a.tol);
@@ -297,12 +299,12 @@ __global__ void __launch_bounds__(kFilterThreads) oc_kernel(const __grid_constan
           else e = r - slo < shi - r ? slo : shi;
         }
         if (threadIdx.x == 0) {
-          w.lo = wlo, w.hi = whi, w.e = e;
-          w.it = wit, w.ilo = ilo, w.ihi = ihi, w.done = wdone || wit >= a.max_iter;
+          w.lo = wlo, w.hi = whi, w.plo = plo, w.phi = phi, w.e = e;
+          w.it = wit, w.done = wdone || wit >= a.max_iter;
         }
       }
       __syncthreads();
-      wlo = w.lo, whi = w.hi, wit = w.it, ilo = w.ilo, ihi = w.ihi;
+      wlo = w.lo, whi = w.hi, plo = w.plo, phi = w.phi, wit = w.it;
       const double e = w.e;
       if (w.done) {
         known = true;
@@ -330,22 +332,25 @@ __global__ void __launch_bounds__(kFilterThreads) oc_kernel(const __grid_constan
       if (!(wlo > 0.0 && whi < 1.0e12)) known = false;
       if (known && wlo != A && !eval(wlo, &vl)) return;
       if (known && whi != B && !eval(whi, &vh)) return;
-      // halvings with the last upper end's volume: the first of them counts
-      if (known && ihi < 60 && whi == ldexp(1.0e12, -(ihi + 1)) && ihi > 0) {
-        double v;
-        if (!eval(2.0 * whi, &v)) return;
-        if (v == vh) known = false;
-      }
       if (known) {
         const double el = fabs(vl - a.target), eh = fabs(vh - a.target);
-        const bool low = el < eh || (el == eh && ilo < ihi);
-        best_err = low ? el : eh;
-        best_lam = low ? wlo : whi;
-        best_vol = low ? vl : vh;
-        lo = wlo;
-        hi = whi;
-        it = wit;
-        done = true;
+        const bool low = el < eh;
+        // the first of equal errors counts: the end is the answer only if the
+        // path's end before it on that side (none: 0 or 1e12) has another volume
+        const double prev = low ? plo : phi;
+        double v = NAN;
+        if (prev > 0.0 && prev < 1.0e12 && !eval(prev, &v)) return;
+        if (el == eh || v == (low ? vl : vh)) {
+          known = false;
+        } else {
+          best_err = low ? el : eh;
+          best_lam = low ? wlo : whi;
+          best_vol = low ? vl : vh;
+          lo = wlo;
+          hi = whi;
+          it = wit;
+          done = true;
+        }
       }
     }
     if (!known) {

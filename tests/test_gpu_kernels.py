@@ -324,6 +324,28 @@ def test_oc_bisection_ties_keep_the_first_step(P, max_iter):
     assert st[0] == best and st[5] == lo and st[6] == hi
 
 
+# A plateau between two evaluations of the walk: the volumes of the path's last end
+# and of an end before it are equal although no evaluation repeated one, and the
+# first of them counts.  (No filter: rmin < 1.)  Upper and lower end.
+@pytest.mark.parametrize("x,q,count,move,beta,target,max_iter,want", [
+    ((0.75, 0.5), (0.5, 1.0), (4, 20), 0.01, 1.0, 13.241930182593716, 80, 0.9094947017729282),
+    ((0.25, 0.75, 0.25), (1.0, 0.5, 0.5), (4, 1, 4), 0.05, 1.0, 2.58963145503766, 60, 0.4547473508864641)])
+def test_oc_walk_keeps_the_first_of_a_plateau(P, x, q, count, move, beta, target, max_iter, want):
+    from pytopo3d_b200.oc_update import OCWorkspace, oc_update_flat
+    from pytopo3d_b200._tensors import to_flat, vec
+
+    x, q = np.repeat(x, count)[None, :, None], np.repeat(q, count)[None, :, None]
+    dc, dv, none = -q * q, np.ones_like(x), np.zeros(x.shape, bool)
+    Ho, Hso = O.build_filter(x.size, 1, 1, 0.9)
+    steps, best, lo, hi = _oracle_bisection((x, dc, dv, move, target, Ho, Hso, beta, 0.5, ~none, none, none), max_iter, 0.3)
+    assert best == want
+    H, Hs = P.build_filter(x.size, 1, 1, 0.9)
+    xf = to_flat(x)
+    st = oc_update_flat(H, xf, to_flat(dc), to_flat(dv), vec(Hs), None, None, move, target, beta, 0.5,
+                        torch.empty_like(xf), torch.empty_like(xf), OCWorkspace(H), max_iter, 0.3).cpu().numpy()
+    assert (int(st[2]), st[0], st[5], st[6]) == (steps, best, lo, hi)
+
+
 def test_expired_barrier_wait_reaches_the_host(P, golden):
     """Every grid-barrier wait of the OC kernel is bounded.  The wait-expiry hook
     makes the barrier wait for a block that never arrives, with a short poll
