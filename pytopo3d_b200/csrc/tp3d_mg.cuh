@@ -470,17 +470,6 @@ __device__ __forceinline__ double gj_shift(const double* __restrict__ D, int n, 
   return (attempt == 1 ? 1e-12 : (attempt == 2 ? 1e-9 : 1e-6)) * m;
 }
 
-// 1 / p by Newton's iteration on the reciprocal from its FP32 rounding (the
-// relative error squares each time: 2^-24, 2^-48, then the FP64 rounding): the
-// division's latency is a third of the chain of pivots.
-__device__ __forceinline__ double gj_rcp(double p) {
-  if (!(p > 1e-30 && p < 1e30)) return 1.0 / p;
-  double r = (double)__frcp_rn((float)p);
-#pragma unroll
-  for (int k = 0; k < 2; ++k) r = fma(r, fma(-p, r, 1.0), r);
-  return r;
-}
-
 // Pivots [32 kb, 32 kb + 32) of the elimination: block (J, I) of the grid writes
 // the 32 x 32 tile (I, J) of `out` from `in`; after the last block `out` holds
 // the inverse (and out32, if given, its rounding).  Rows and columns past n are
@@ -491,8 +480,8 @@ __device__ __forceinline__ double gj_rcp(double p) {
 // the tile (k, k) and multiplying, A_IJ - A_Ik P A_kJ, is shorter but loses
 // accuracy with the condition of that tile: on nearly singular binary designs CG
 // took 10000 iterations instead of 1500.)
-// The pivots in series bound it, about 12 us a step with the launch: 64 us at
-// n = 135, 143 us at 336, 249 us at 480.  One block holding the whole matrix took
+// The pivots in series bound it, 11 us a step at n = 135 and 336 and 16 us at 480:
+// 53, 123 and 233 us in all.  One block holding the whole matrix took
 // 235 us at n = 135 (entries in registers) and 8.5 ms at n = 336 (entries in L2,
 // two barriers and 900 KB of traffic per pivot).
 __global__ void __launch_bounds__(256) gj_block_step_kernel(int n, int kb, const double* __restrict__ in,
@@ -532,7 +521,7 @@ __global__ void __launch_bounds__(256) gj_block_step_kernel(int n, int kb, const
       __syncthreads();
       const double p = rowA[buf][k], ga = rowA[buf][tx], gb = rowB[buf][tx];
       bad = bad || !(p > 0.0);
-      const double pk = gj_rcp(p);
+      const double pk = 1.0 / p;
 #pragma unroll
       for (int r = 0; r < 4; ++r) {
         const double f = colA[buf][ty + 8 * r] * pk, h = colC[buf][ty + 8 * r] * pk;
