@@ -441,6 +441,7 @@ __global__ void __launch_bounds__(kFilterThreads) oc_kernel(const __grid_constan
       a.stats[5] = lo;
       a.stats[6] = hi;
       a.stats[7] = have ? best_err : NAN;
+      a.bar.count[3] = (unsigned int)pass;  // volume evaluations, for tests (cleared with the barrier words)
     }
   }
 }

@@ -25,6 +25,11 @@ class OCWorkspace:
         self.scratch = torch.empty(n, dtype=torch.uint8, device=device())
         self.stats = torch.empty(8, dtype=torch.float64, device=device())
 
+    def evaluations(self) -> int:
+        """Volume evaluations of the last update (waits for it): the fourth of the
+        kernel's 32-bit words in the last 256 bytes of the scratch."""
+        return int(self.scratch[-256:].view(torch.int32)[3])
+
 
 def oc_update_flat(H: ConeFilter, x, dc_dx, dv_dx, Hs, solid, void, move, target, beta, eta,
                    x_new, rho_new, ws: OCWorkspace, max_bisection_iterations=80,

@@ -374,14 +374,15 @@ def test_expired_barrier_wait_reaches_the_host(P, golden):
 
 
 # The OC kernel walks the reference's path from a few evaluations (secant steps
-# between halvings of the multiplier): sizes at the edges of its 32 x 8 tiles and
-# of its planes per block, every filter radius class, multipliers far below the
-# first probe (spread: log-normal sensitivities), and targets that no multiplier
-# reaches from either side (the walk is left for the ordinary steps).
+# between halvings of the multiplier): sizes at the edges of its 32 x 8 x 8 tiles,
+# more tiles than blocks that fit the GPU (900), every filter radius class,
+# multipliers far below the first probe (spread: log-normal sensitivities), and
+# targets that no multiplier reaches from either side (the walk is left for the
+# ordinary steps).
 @pytest.mark.parametrize("dims,rmin,spread,frac", [
     ((8, 32, 7), 1.2, 1.0, 0.3), ((9, 33, 3), 2.3, 4.0, 0.4), ((17, 5, 21), 3.6, 1.0, 0.5), ((16, 31, 2), 4.4, 8.0, 0.3),
-    ((12, 14, 9), 5.5, 0.5, 0.45), ((13, 8, 15), 6.9, 2.0, 0.35), ((8, 9, 6), 0.9, 3.0, 0.3), ((24, 12, 13), 1.5, 2.0, -1.0),
-    ((24, 12, 13), 2.9, 2.0, 2.0)])
+    ((12, 14, 9), 5.5, 0.5, 0.45), ((13, 8, 15), 6.9, 2.0, 0.35), ((8, 9, 6), 0.9, 3.0, 0.3), ((2400, 2, 17), 1.5, 1.0, 0.4),
+    ((24, 12, 13), 1.5, 2.0, -1.0), ((24, 12, 13), 2.9, 2.0, 2.0)])
 def test_oc_walk_matches_oracle_path(P, dims, rmin, spread, frac):
     from pytopo3d_b200.oc_update import OCWorkspace, oc_update_flat
     from pytopo3d_b200._tensors import from_flat, to_flat, to_flat_mask, vec
@@ -412,8 +413,12 @@ def test_oc_walk_matches_oracle_path(P, dims, rmin, spread, frac):
     H, Hs = P.build_filter(nx, ny, nz, rmin)
     xf = to_flat(x)
     xn, rn = torch.empty_like(xf), torch.empty_like(xf)
+    ws = OCWorkspace(H)
     st = oc_update_flat(H, xf, to_flat(dc), to_flat(dv), vec(Hs), to_flat_mask(solid), to_flat_mask(void), move, target,
-                        beta, eta, xn, rn, OCWorkspace(H)).cpu().numpy()
+                        beta, eta, xn, rn, ws).cpu().numpy()
+    # the walk's evaluations (9 to 15 measured) and not the path's; below every
+    # candidate it is left at once, and every step but the first is evaluated
+    assert ws.evaluations() >= steps if frac < 0.0 else ws.evaluations() <= 20
     assert int(st[2]) == steps
     assert st[0] == best and st[5] == lo and st[6] == hi
     # the same multiplier: candidates to rounding, filtered densities to the filter's 1e-12
