@@ -21,6 +21,31 @@ struct ColsEntry {
 std::mutex g_cols_mu;
 std::map<std::pair<int, unsigned long long>, ColsEntry> g_cols;
 
+// One allocation for both arrays, on a stream of its own and in relaxed capture
+// mode: the first call for a radius may come inside a stream capture.
+int upload_cols(const std::vector<int2>& dxy, const std::vector<double>& w, ColsEntry* e) {
+  const size_t wbytes = w.size() * sizeof(double), dbytes = dxy.size() * sizeof(int2);
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  TP3D_CHECK(cudaThreadExchangeStreamCaptureMode(&mode));
+  char* base = nullptr;
+  cudaStream_t up = nullptr;
+  cudaError_t err = cudaMalloc(&base, wbytes + dbytes);
+  if (err == cudaSuccess) err = cudaStreamCreateWithFlags(&up, cudaStreamNonBlocking);
+  if (err == cudaSuccess) err = cudaMemcpyAsync(base, w.data(), wbytes, cudaMemcpyHostToDevice, up);
+  if (err == cudaSuccess) err = cudaMemcpyAsync(base + wbytes, dxy.data(), dbytes, cudaMemcpyHostToDevice, up);
+  if (up) {
+    const cudaError_t done = cudaStreamSynchronize(up);
+    if (err == cudaSuccess) err = done;
+    cudaStreamDestroy(up);
+  }
+  if (err != cudaSuccess && base) cudaFree(base);
+  cudaThreadExchangeStreamCaptureMode(&mode);
+  TP3D_CHECK(err);
+  e->w = reinterpret_cast<double*>(base);
+  e->dxy = reinterpret_cast<int2*>(base + wbytes);
+  return TP3D_OK;
+}
+
 }  // namespace
 
 // Taps: integer offsets d with rmin - |d| > 1e-9 and weight rmin - sqrt(|d|^2)
@@ -47,14 +72,9 @@ int filter_cols_for(double rmin, FilterCols* out) {
     std::vector<double> w((size_t)ncols * (2 * Z + 1));
     filter_columns_build(rmin, Z, dxy.data(), w.data());
     ColsEntry e;
-    e.ncols = (int)dxy.size();
+    e.ncols = ncols;
     e.Z = Z;
-    if (cudaMalloc(&e.dxy, dxy.size() * sizeof(int2)) != cudaSuccess) return TP3D_ERR_CUDA;
-    if (cudaMalloc(&e.w, w.size() * sizeof(double)) != cudaSuccess) return TP3D_ERR_CUDA;
-    if (cudaMemcpy(e.dxy, dxy.data(), dxy.size() * sizeof(int2), cudaMemcpyHostToDevice) != cudaSuccess)
-      return TP3D_ERR_CUDA;
-    if (cudaMemcpy(e.w, w.data(), w.size() * sizeof(double), cudaMemcpyHostToDevice) != cudaSuccess)
-      return TP3D_ERR_CUDA;
+    if (int rc = upload_cols(dxy, w, &e)) return rc;
     it = g_cols.emplace(key, e).first;
   }
   out->dxy = it->second.dxy;

@@ -84,6 +84,19 @@ def test_filter_sums_keep_their_order(P, dims, rmin):
     np.testing.assert_array_equal(rf, want)
 
 
+def test_first_filter_call_of_a_radius_inside_a_capture(P):
+    """The radius's column table goes up during the call; a captured first call is
+    as good as any other (2.5625 is used nowhere else)."""
+    nx, ny, nz, r = 9, 7, 5, 2.5625
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        _, Hs = P.build_filter(nx, ny, nz, r)
+    graph.replay()
+    torch.cuda.synchronize()
+    _, Hso = O.build_filter(nx, ny, nz, r)
+    np.testing.assert_allclose(Hs.cpu().numpy(), Hso, rtol=1e-14, atol=0)
+
+
 def test_projection_matches_golden(P, golden):
     nx, ny, nz, r = golden["bpd_dims"]
     H, Hs = P.build_filter(int(nx), int(ny), int(nz), float(r))
