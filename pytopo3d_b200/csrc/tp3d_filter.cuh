@@ -14,10 +14,11 @@
 // residual of 1e-10, which the sensitivities of nearly void elements amplify, and a
 // change of one unit in the last place of the design moves the design three steps
 // later by more than 2e-9 on 6 of 40 random grids with protected voids.  Ring sums
-// per plane marched along z round differently and were taken back for that: filter
-// and projection 17 us at 128x64x64 (rmin 3) and 169 us at 256x128x128 (rmin 4.5)
-// against 23 and 294 us here, OC update (the same evaluations) 385 and 3091 us
-// against 330 and 4446.
+// per plane marched along z were taken back for that, and for their error: 1.1e-15
+// against 1.4e-16 here (filter, projection and chain rule at 128x64x64, rmin 3,
+// relative to plain 64-bit sums).  They took 17 us for filter and projection there
+// and 169 us at 256x128x128 (rmin 4.5) against 23 and 294 us here, the OC update
+// (the same evaluations) 385 and 3091 us against 330 and 4446.
 #pragma once
 
 #include "tp3d_common.cuh"

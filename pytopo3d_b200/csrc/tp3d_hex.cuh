@@ -592,7 +592,7 @@ __global__ void __launch_bounds__(kRestrictResidThreads) restrict_resid_kernel(
 
 // x_f[i] += sum_I P[i,I] x_c[I] on free fine DOFs.  A fine node takes 1, 2, 4
 // or 8 coarse nodes (weights 1 or 1/2 per axis), read as a fixed 2x2x2 block
-// with zero weights for the absent ones.  Grid: plane_grid(FX*FY, FZ).
+// with zero weights for the absent ones.  (For the cycles of several levels in one launch.)
 template <typename T, class Ld = LdRO>
 __device__ __forceinline__ void prolong_node(const Grid& gf, const Grid& gc, const T* __restrict__ xc,
                                              const uint8_t* __restrict__ fixf, T* xf, int ix, int iy, int iz) {
@@ -635,7 +635,7 @@ __device__ __forceinline__ void prolong_node(const Grid& gf, const Grid& gc, con
 // coarse nodes of weight 0 (even x or z) are not read at all: 13.5 values per pair
 // on average in place of 48 (prolong_node's fixed 2x2x2 blocks): 31 us on the fine
 // level of 256x128x128, 64 before.  The sums' order and rounding are prolong_node's.
-// Grid: plane_grid((FX) * pairs along y, FZ).
+// Grid: plane_grid(FX * pairs along y, FZ).
 inline int prolong_pairs(const Grid& gf) { return gf.ny / 2 + 1; }
 
 template <typename T>

@@ -97,6 +97,9 @@ struct __align__(16) Pack {
 
 // u += alpha p; r -= alpha q; partials of ||r||^2 (with fin_count, the last
 // block applies op to st)
+// A thread sums neighbouring values into ||r||^2, so that sum (read by the stop test
+// and the reliable update's trigger only) is rounded in another order than with a
+// value per access; the vectors are not.
 // With fs.x0 set, also the V-cycle's first smoothing step from the new
 // residual (pointwise: x0 = w dinv r, d = x0), as smooth_zero_kernel computes it.
 template <typename T>
